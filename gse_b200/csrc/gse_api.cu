@@ -158,11 +158,11 @@ struct gse_context {
   int nbins2 = 0;
   int* d_bkey = nullptr;
   int* d_btmp = nullptr;
+  double* d_basis = nullptr;  // FP64 form: spread weights' basis of the sorted atoms
   int* d_bcounts = nullptr;
   int* d_bstart = nullptr;
   int* d_blstart = nullptr;  // mixed form: tile-local bin starts of the scan
   int* d_btiles = nullptr;
-  unsigned* d_qmax = nullptr;
   // Green's function table of the context's own solve (sigma2, box)
   void* d_gtab = nullptr;
   bool gtab_valid = false;
@@ -318,6 +318,8 @@ gse_status_t ensure_atoms(gse_context_t* c, int n) {
   cudaFree(c->d_force);
   cudaFree(c->d_bkey);
   cudaFree(c->d_btmp);
+  cudaFree(c->d_basis);
+  c->d_basis = nullptr;
   c->d_xyzq = c->d_sorted = nullptr;
   c->d_perm = nullptr;
   c->d_force = nullptr;
@@ -330,6 +332,7 @@ gse_status_t ensure_atoms(gse_context_t* c, int n) {
   CU(cudaMalloc(&c->d_force, 3 * cap * sizeof(double)));
   CU(cudaMalloc(&c->d_bkey, cap * sizeof(int)));
   CU(cudaMalloc(&c->d_btmp, cap * sizeof(int)));
+  if (c->fp64) CU(cudaMalloc(&c->d_basis, cap * kBasis64 * sizeof(double)));
   c->atom_cap = cap;
   return GSE_OK;
 }
@@ -354,17 +357,25 @@ gse_status_t stage_atoms(gse_context_t* c, int n, const void* xyzq, const void**
   return GSE_OK;
 }
 
+// The brick-tiled spread and gather take this stencil and grid.
+template <typename CT>
+bool tiled_ok(const gse_context_t* c, const Stencil<CT>& s) {
+  return spread_tiled_supported<CT>(s) && c->p.size_x >= kMinTiledGrid &&
+         c->p.size_y >= kMinTiledGrid && c->p.size_z >= kMinTiledGrid;
+}
+
 // Stable counting sort of the atoms into c->d_sorted / c->d_perm by
 // (z cell, y cell, x bin) of their stencil centres; c->d_bstart holds the bin
 // offsets afterwards.
 // clear_fixed: the counting kernel also clears the mixed form's int64 grid.
+// basis: FP64 form, the tiled spread with this stencil follows (its weights'
+// basis is formed with the sort).
 template <typename CT>
 gse_status_t bin_atoms(gse_context_t* c, int n, const void* dx, const Stencil<CT>& s,
-                       bool clear_fixed = false) {
+                       bool clear_fixed = false, bool basis = false) {
   typedef typename Vec4<CT>::type V;
   StageTimer tm(c, GSE_STAGE_BIN);
-  BinScratch w{c->d_bkey, c->d_bcounts, c->d_bstart, c->d_btiles, c->d_btmp, c->d_qmax,
-               c->d_badmap};
+  BinScratch w{c->d_bkey, c->d_bcounts, c->d_bstart, c->d_btiles, c->d_btmp, c->d_badmap};
   // mixed: count, a tile-local scan and the placement that applies the tile
   // offsets (the counts stay zero between calls); FP64: count, three scan
   // passes and a stable placement in two kernels
@@ -376,17 +387,14 @@ gse_status_t bin_atoms(gse_context_t* c, int n, const void* dx, const Stencil<CT
       w.clear_n = c->size;
     }
   }
+  if constexpr (sizeof(CT) == 8) {
+    if (basis && tiled_ok<CT>(c, s))
+      w.basis = SpreadBasis{{s.h[0], s.h[1], s.h[2]}, s.inv_2s2, s.pref, s.nst[0], c->d_basis};
+  }
   c->launches += c->fp64 ? (n > 0 ? 6 : 3) : (n > 0 ? 3 : 2);
   CU(launch_bin_sorted<CT>((const V*)dx, n, c->bl, s.inv_h[0], s.inv_h[1], s.inv_h[2], w,
                            (V*)c->d_sorted, c->d_perm, c->stream));
   return GSE_OK;
-}
-
-// Size the scatter buffers for stencil width W (once per width).
-template <typename CT>
-bool tiled_ok(const gse_context_t* c, const Stencil<CT>& s) {
-  return spread_tiled_supported<CT>(s) && c->p.size_x >= kMinTiledGrid &&
-         c->p.size_y >= kMinTiledGrid && c->p.size_z >= kMinTiledGrid;
 }
 
 // Spread into c->d_rho.  `presorted`: c->d_sorted / d_bstart already hold the
@@ -402,13 +410,13 @@ gse_status_t do_spread(gse_context_t* c, int n, const void* dx, const double box
   typedef typename Vec4<CT>::type V;
   const Stencil<CT> s = stencil_of<CT>(c, box, sigma, rcut, false, normalize);
   if (!normalize && tiled_ok<CT>(c, s)) {
-    if (!presorted) TRY(bin_atoms<CT>(c, n, dx, s));
+    if (!presorted) TRY(bin_atoms<CT>(c, n, dx, s, false, c->fp64));
     StageTimer tm(c, GSE_STAGE_SPREAD);
-    if (c->fp64) {
+    if constexpr (sizeof(CT) == 8) {
       c->launches += 1;
-      CU(launch_spread_tiled<CT>((const V*)c->d_sorted, c->d_bstart, c->d_qmax, c->bl, s,
-                                 (CT*)c->d_rho, c->stream));
-    } else if constexpr (sizeof(CT) == 4) {
+      CU(launch_spread64(c->d_basis, c->d_bstart, c->bl, s, (double*)c->d_rho,
+                         c->stream));
+    } else {
       const bool defer = defer_rho && c->own_fft;
       c->launches += defer ? 1 : 2;
       CU(launch_spread_scatter((const float4*)c->d_sorted, c->d_bstart, c->bl, s, c->d_fixed,
@@ -904,7 +912,6 @@ gse_status_t gse_create(const gse_params_t* params, gse_context_t** out) {
   if (!c->fp64) CUC(cudaMalloc(&c->d_blstart, sizeof(int) * c->nbins2));
   CUC(cudaMalloc(&c->d_bstart, sizeof(int) * (c->nbins2 + 1)));
   CUC(cudaMalloc(&c->d_btiles, sizeof(int) * (c->nbins2 / 4096 + 2)));
-  CUC(cudaMalloc(&c->d_qmax, sizeof(unsigned)));
   CUC(cudaMalloc(&c->d_partials, sizeof(double) * (kEnergyPartials + 1)));
   CUC(cudaMemset(c->d_partials, 0, sizeof(double) * (kEnergyPartials + 1)));
   CUC(cudaMalloc(&c->d_scalars, sizeof(double) * 16));
@@ -954,11 +961,11 @@ gse_status_t gse_destroy(gse_context_t* c) {
   cudaFree(c->d_force);
   cudaFree(c->d_bkey);
   cudaFree(c->d_btmp);
+  cudaFree(c->d_basis);
   cudaFree(c->d_bcounts);
   cudaFree(c->d_blstart);
   cudaFree(c->d_bstart);
   cudaFree(c->d_btiles);
-  cudaFree(c->d_qmax);
   cudaFree(c->d_gtab);
   cudaFree(c->d_adj);
   cudaFree(c->d_partials);
@@ -1102,7 +1109,8 @@ gse_status_t forward_body(gse_context_t* c, int n, const void* xyzq, double* ene
   // are timed)
   bool zeroed = false;
   if (c->fp64) {
-    TRY(bin_atoms<double>(c, n, dx, stencil_of<double>(c, box.v, c->sigma1, c->rcut1, false, false)));
+    TRY(bin_atoms<double>(c, n, dx, stencil_of<double>(c, box.v, c->sigma1, c->rcut1, false, false),
+                          false, true));
   } else {
     const Stencil<float> s = stencil_of<float>(c, box.v, c->sigma1, c->rcut1, false, false);
     zeroed = !c->timing && tiled_ok<float>(c, s);
@@ -1643,7 +1651,8 @@ gse_status_t gse_adjoint(gse_context_t* c, int n, const void* xyzq, double dLdE,
   const double gE_ch3 = dLdE * c->p.ccelec * h3;
   // forward grids, recomputed from the inputs (rho -> phi)
   if (c->fp64)
-    TRY(bin_atoms<double>(c, n, dxq, stencil_of<double>(c, box.v, c->sigma1, c->rcut1, false, false)));
+    TRY(bin_atoms<double>(c, n, dxq, stencil_of<double>(c, box.v, c->sigma1, c->rcut1, false, false),
+                          false, true));
   else
     TRY(bin_atoms<float>(c, n, dxq, stencil_of<float>(c, box.v, c->sigma1, c->rcut1, false, false)));
   if (c->fp64)

@@ -186,7 +186,6 @@ cudaError_t launch_ewald_direct(const double4* xyzq, int n, const EwdGeom& g, Ew
   b.start = w.start;
   b.tile_sums = w.tile_sums;
   b.tmp = w.tmp;
-  b.qmax_bits = nullptr;
   e = launch_bin_scan_place<double>(xyzq, n, g.ncell, b, w.sorted, w.perm, st);
   if (e != cudaSuccess) return e;
   k_ewd_pairs<<<g.ncell, kEwdThreads, 0, st>>>(w.sorted, w.perm, w.start, g, ex_start, ex_idx,

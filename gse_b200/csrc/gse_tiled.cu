@@ -4,15 +4,10 @@
 //            of their stencil centre round(x/h) mod M; the FP64 form keeps the
 //            original order within a bin so that its sums run in a fixed
 //            order, the mixed form's integer sums need no order.
-//  spread    CpuGaussCharge::spreadChargeToGrid (CpuGaussCharge.cpp:235-384).
-//            FP64 form: output-stationary.  A CTA owns a kTX x kTY x TZ block
-//            of the grid; each thread owns one (x, y) column of it with TZ
-//            accumulators in registers.  The atoms whose (2n+1)^3 cube reaches
-//            the block stream through shared memory in chunks; each warp keeps
-//            the ones that touch its 8 x 4 column patch and adds their 2n+1 z
-//            weights into its registers.  No atomics; every grid point is
-//            written once.  Mixed form: atom-stationary scatter into an int32
-//            shared brick tile, added into an int64 grid (scatter_brick).
+//  spread    CpuGaussCharge::spreadChargeToGrid (CpuGaussCharge.cpp:235-384),
+//            mixed form: atom-stationary scatter into an int32 shared brick
+//            tile, added into an int64 grid (scatter_brick).  The FP64 form's
+//            output-stationary spread is in gse_spread64.cu.
 //  gather    CpuGaussCharge::interpolateLoop (CpuGaussCharge.cpp:105-172): a
 //            CTA owns the atoms of a kGX x kGY x kGZ-cell brick and stages the
 //            potential of the brick plus its n-cell halo in shared memory;
@@ -36,8 +31,7 @@ namespace gse {
 template <typename CT>
 __global__ void k_bin_count(const typename Vec4<CT>::type* __restrict__ xyzq, int n, BinLayout b,
                             CT inv_hx, CT inv_hy, CT inv_hz, int* __restrict__ key,
-                            int* __restrict__ counts, unsigned* __restrict__ qmax_bits,
-                            int* __restrict__ bad, long long* __restrict__ clear,
+                            int* __restrict__ counts, int* __restrict__ bad, long long* __restrict__ clear,
                             long long clear_n, int* __restrict__ rank) {
   pdl_trigger();
   if (clear) {
@@ -47,12 +41,10 @@ __global__ void k_bin_count(const typename Vec4<CT>::type* __restrict__ xyzq, in
       reinterpret_cast<int4*>(clear)[i] = make_int4(0, 0, 0, 0);
     if ((clear_n & 1) && first == 0) clear[clear_n - 1] = 0;
   }
-  float qm = 0.f;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const auto a = xyzq[i];
     if (bad && !(isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w)))
       *bad = kFlagNonFinite;  // the bin below is still in range (wrap1 of any int)
-    qm = fmaxf(qm, fabsf((float)a.w));
     const int cx = wrap1(centre_cell(a.x, inv_hx), b.M[0]);
     const int cy = wrap1(centre_cell(a.y, inv_hy), b.M[1]);
     const int cz = wrap1(centre_cell(a.z, inv_hz), b.M[2]);
@@ -62,19 +54,6 @@ __global__ void k_bin_count(const typename Vec4<CT>::type* __restrict__ xyzq, in
     // form's consumers are order-free), so the placement needs no atomics
     const int r = atomicAdd(&counts[k], 1);
     if (rank) rank[i] = r;
-  }
-  if (!qmax_bits) return;  // uniform
-  // block maximum first: one atomic per block, not per warp, on the single
-  // address (same-address atomics serialise)
-  __shared__ float wmax[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) qm = fmaxf(qm, __shfl_xor_sync(0xffffffffu, qm, o));
-  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = qm;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) qm = fmaxf(qm, wmax[w]);
-    // non-negative floats order like their bit patterns (NaN compares largest)
-    atomicMax(qmax_bits, __float_as_uint(qm));
   }
 }
 
@@ -203,286 +182,40 @@ __global__ void __launch_bounds__(256)
   if (gtid == 0) start[nb] = off[ntiles - 1] + tile_sums[ntiles - 1];
 }
 
-// Stable placement: an atom's rank in its bin is the number of bin members
-// with a smaller original index.
-template <typename CT>
-__global__ void k_bin_place_stable(const typename Vec4<CT>::type* __restrict__ xyzq, int n,
+// Stable placement (FP64 form): an atom's rank in its bin is the number of bin
+// members with a smaller original index.
+__global__ void k_bin_place_stable(const double4* __restrict__ xyzq, int n,
                                    const int* __restrict__ key, const int* __restrict__ start,
-                                   const int* __restrict__ tmp,
-                                   typename Vec4<CT>::type* __restrict__ sorted,
-                                   int* __restrict__ perm) {
+                                   const int* __restrict__ tmp, double4* __restrict__ sorted,
+                                   int* __restrict__ perm, BinLayout b, double3 inv_h,
+                                   SpreadBasis sb) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int k = key[i];
     const int s = start[k], e = start[k + 1];
     int r = 0;
     for (int j = s; j < e; j++) r += (tmp[j] < i);
-    sorted[s + r] = xyzq[i];
+    const double4 a = xyzq[i];
+    sorted[s + r] = a;
     perm[s + r] = i;
-  }
-}
-
-// ===========================================================================
-// Spread
-// ===========================================================================
-// Accumulator / z-weight types of the spread.  FP64 form: double
-// accumulators and weights.  Mixed form: the z weights are int32 fixed point
-// (kWzBits fraction bits), the (x, y) factor t = q pref wx wy is rounded to
-// int32 with a per-launch scale, and each product t_int * wz_int is added
-// exactly into an int64 accumulator (one mad.wide.s32), so the grid sum is
-// independent of the order of the contributions.
-template <typename CT> struct SpreadTypes;
-template <> struct SpreadTypes<double> {
-  typedef double Acc;
-  typedef double Wz;
-  typedef double T;
-};
-template <> struct SpreadTypes<float> {
-  typedef long long Acc;
-  typedef int Wz;
-  typedef int T;
-};
-constexpr int kWzBits = 26;
-
-__device__ __forceinline__ double madd(double t, double w, double a) { return fma(t, w, a); }
-__device__ __forceinline__ long long madd(int t, int w, long long a) {
-  return a + (long long)t * (long long)w;
-}
-
-template <typename CT>
-struct SpreadRec {
-  int s[3];                                // first stencil cell relative to the block origin
-  CT qp;                                   // q * (2 pi sigma^2)^(-3/2)
-  CT w[2][kWPad];                          // x and y weights
-  typename SpreadTypes<CT>::Wz wz[kWPad];  // z weights (fixed point in the mixed form)
-};
-
-// acc[OZ + k] += t * wz[k] for the k that land inside the block (compile-time
-// indices, so the accumulators stay in registers).
-template <typename A, typename T, typename WZ, int TZ, int W, int OZ>
-__device__ __forceinline__ void add_column(A (&acc)[TZ], T t, const WZ (&wz)[kWPad]) {
+    if (sb.out) {
+      const double x[3] = {a.x, a.y, a.z}, ih[3] = {inv_h.x, inv_h.y, inv_h.z};
+      double v[kBasis64];
 #pragma unroll
-  for (int k = 0; k < W; k++) {
-    if (OZ + k >= 0 && OZ + k < TZ) acc[OZ + k] = madd(t, wz[k], acc[OZ + k]);
-  }
-}
-
-#define GSE_ZC(i) \
-  case i: add_column<A, T, WZ, TZ, W, (i) - (W - 1)>(acc, t, wz); break;
-#define GSE_ZC8(i) GSE_ZC(i) GSE_ZC(i + 1) GSE_ZC(i + 2) GSE_ZC(i + 3) GSE_ZC(i + 4) GSE_ZC(i + 5) \
-  GSE_ZC(i + 6) GSE_ZC(i + 7)
-
-// The block-relative z offset oz is the same for the whole warp: one
-// indirect branch selects the unrolled case.
-template <typename A, typename T, typename WZ, int TZ, int W>
-__device__ __forceinline__ void add_column_dispatch(int oz, A (&acc)[TZ], T t,
-                                                    const WZ (&wz)[kWPad]) {
-  static_assert(TZ + W - 1 <= 96, "z dispatch covers 96 offsets");
-  switch (oz + W - 1) {
-    GSE_ZC8(0) GSE_ZC8(8) GSE_ZC8(16) GSE_ZC8(24) GSE_ZC8(32) GSE_ZC8(40)
-    GSE_ZC8(48) GSE_ZC8(56) GSE_ZC8(64) GSE_ZC8(72) GSE_ZC8(80) GSE_ZC8(88)
-    default: break;
-  }
-}
-#undef GSE_ZC8
-#undef GSE_ZC
-
-// 1-D weights w[j] = exp(-(dc + (j - n) h)^2 / (2 sigma^2)), j < W = 2n+1,
-// where dc = c h - x is the offset of the stencil centre (the reference's
-// d0 + j h with d0 = (c - n) h - x, CpuGaussCharge.cpp:311-329).  Evaluated
-// outward from the centre by the exact ratio recurrence
-//   w[n+k] = w[n+k-1] ru[k-1],  ru[k] = ru[k-1] exp(-2 h^2/(2 sigma^2)),
-// and the mirror image below the centre.  The decay factor is applied as an
-// unevaluated sum hi + lo so that its rounding does not compound.
-template <typename CT, int W>
-__device__ __forceinline__ void gauss_row(CT dc, CT h, CT inv_2s2, CT dec_hi, CT dec_lo,
-                                          CT (&w)[kWPad]) {
-  constexpr int n = (W - 1) / 2;
-  const CT wc = gexp(mul_rn(mul_rn(-dc, dc), inv_2s2));
-  const CT hh = h * h;
-  CT ru = gexp(-(2 * dc * h + hh) * inv_2s2);   // w[n+1] / w[n]
-  CT rd = gexp(-(hh - 2 * dc * h) * inv_2s2);   // w[n-1] / w[n]
-  w[n] = wc;
-  CT wu = wc, wd = wc;
-#pragma unroll
-  for (int k = 1; k <= n; k++) {
-    wu *= ru;
-    wd *= rd;
-    w[n + k] = wu;
-    w[n - k] = wd;
-    ru = fma(ru, dec_hi, ru * dec_lo);
-    rd = fma(rd, dec_hi, rd * dec_lo);
-  }
-#pragma unroll
-  for (int j = W; j < kWPad; j++) w[j] = (CT)0;
-}
-
-template <typename CT, int TZ, int W>
-__global__ void __launch_bounds__(kSpreadThreads)
-    k_spread_tiled(const typename Vec4<CT>::type* __restrict__ sorted,
-                   const int* __restrict__ start, const unsigned* __restrict__ qmax_bits,
-                   BinLayout b, Stencil<CT> s, Decay<CT> dec, CT* __restrict__ grid) {
-  constexpr int n = (W - 1) / 2;
-  constexpr int CH = sizeof(CT) == 8 ? kSpreadChunk : 2 * kSpreadChunk;
-  constexpr int NT = kSpreadThreads;
-  constexpr bool FIXED = sizeof(CT) == 4;
-  typedef typename Vec4<CT>::type V;
-  typedef typename SpreadTypes<CT>::Acc A;
-  typedef typename SpreadTypes<CT>::T T;
-  typedef typename SpreadTypes<CT>::Wz WZ;
-  __shared__ SpreadRec<CT> rec[CH];
-  __shared__ int chunk_atom[CH];
-  __shared__ short chunk_shift[CH][3];
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, z0 = blockIdx.z * TZ;
-  const int ex = min(kTX, b.M[0] - x0), ey = min(kTY, b.M[1] - y0), ez = min(TZ, b.M[2] - z0);
-  // warp patch: 8 (x) x 4 (y); lane -> one column
-  const int px0 = (warp & 1) * 8, py0 = (warp >> 1) * 4;
-  const int cx = px0 + (lane & 7), cy = py0 + (lane >> 3);
-
-  // mixed form: t is rounded to int32 at 2^st; choose st so that
-  // |q pref| 2^st < 2^31 for every atom of the launch
-  int st = 0;
-  float tscale = 1.f;
-  if (FIXED) {
-    const float qpm = __uint_as_float(*qmax_bits) * fabsf((float)s.pref);
-    st = 30;
-    if (!(qpm < 3.0e38f)) {
-      st = 0;
-    } else {
-      while (st > 0 && qpm * exp2f((float)st) >= 2.0e9f) st--;
-    }
-    tscale = exp2f((float)st);
-  }
-
-  A acc[TZ];
-#pragma unroll
-  for (int z = 0; z < TZ; z++) acc[z] = (A)0;
-
-  // rows (uy, uz) of the relevant region, unwrapped cell coordinates
-  const int ry0 = y0 - n, rz0 = z0 - n;
-  const int nry = ey + 2 * n, nrz = ez + 2 * n;
-  const int nrows = nry * nrz;
-  const int ux_lo = x0 - n, ux_hi = x0 + ex + n;  // [lo, hi)
-
-  for (int rbase = 0; rbase < nrows; rbase += NT) {
-    // --- this thread's row: wrapped x segments -> atom ranges ---
-    const int r = rbase + tid;
-    int seg_a[kMaxSeg], seg_e[kMaxSeg], seg_sh[kMaxSeg];
-    int nseg = 0, cnt = 0, shy = 0, shz = 0;
-    if (r < nrows) {
-      const int uy = ry0 + r % nry, uz = rz0 + r / nry;
-      const int ccy = pmod(uy, b.M[1]), ccz = pmod(uz, b.M[2]);
-      shy = uy - ccy;
-      shz = uz - ccz;
-      const int rowkey = (ccz * b.M[1] + ccy) * b.nbx;
-      int u = ux_lo;
-      while (u < ux_hi && nseg < kMaxSeg) {
-        const int cu = pmod(u, b.M[0]);
-        const int seg_end = min(ux_hi, u + (b.M[0] - cu));  // end of this period
-        const int c1 = cu + (seg_end - u);                  // exclusive cell end
-        const int a0 = start[rowkey + (cu >> b.bxs)];
-        const int a1 = start[rowkey + ((c1 - 1) >> b.bxs) + 1];
-        seg_a[nseg] = a0;
-        seg_e[nseg] = a1;
-        seg_sh[nseg] = u - cu;
-        cnt += a1 - a0;
-        nseg++;
-        u = seg_end;
+      for (int d = 0; d < 3; d++) {
+        const int c = centre_cell(x[d], ih[d]);
+        // offset of the centre point, from the first point's offset as the reference
+        // rounds it (d0 = (c - n) h - x, CpuGaussCharge.cpp:311-329)
+        const double h = sb.h[d], hh = h * h;
+        const double dc = sub_rn(mul_rn((double)(c - sb.nst), h), x[d]) + (double)sb.nst * h;
+        const double wc = exp(mul_rn(mul_rn(-dc, dc), sb.inv_2s2));
+        v[3 * d] = d == 0 ? a.w * sb.pref * wc : wc;
+        v[3 * d + 1] = exp(-(2 * dc * h + hh) * sb.inv_2s2);
+        v[3 * d + 2] = exp(-(hh - 2 * dc * h) * sb.inv_2s2);
+        if (d == 0) v[9] = (double)wrap1(c, b.M[0]);
       }
-    }
-    int total;
-    const int pos0 = block_exclusive_scan(cnt, &total);
-    for (int sub = 0; sub < total; sub += CH) {
-      // --- copy this thread's atoms with group positions in [sub, sub+CH) ---
-      int p = pos0;
-      for (int g = 0; g < nseg; g++) {
-        for (int j = seg_a[g]; j < seg_e[g]; j++, p++) {
-          if (p >= sub && p < sub + CH) {
-            chunk_atom[p - sub] = j;
-            chunk_shift[p - sub][0] = (short)seg_sh[g];
-            chunk_shift[p - sub][1] = (short)shy;
-            chunk_shift[p - sub][2] = (short)shz;
-          }
-        }
-      }
-      __syncthreads();
-      const int cntc = min(CH, total - sub);
-      // --- per-atom records ---
-      for (int i = tid; i < cntc; i += NT) {
-        const V a = sorted[chunk_atom[i]];
-        const CT pos[3] = {a.x, a.y, a.z};
-        const int org[3] = {x0, y0, z0};
-        CT wz[kWPad];
+      double2* o = reinterpret_cast<double2*>(sb.out + (long long)(s + r) * kBasis64);
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-          const int c = centre_cell(pos[d], s.inv_h[d]);
-          const CT dc = sub_rn(mul_rn((CT)c, s.h[d]), pos[d]);
-          CT w[kWPad];
-          gauss_row<CT, W>(dc, s.h[d], s.inv_2s2, dec.hi[d], dec.lo[d], w);
-          if (d < 2) {
-#pragma unroll
-            for (int j = 0; j < kWPad; j++) rec[i].w[d][j] = w[j];
-          } else {
-#pragma unroll
-            for (int j = 0; j < kWPad; j++) wz[j] = w[j];
-          }
-          rec[i].s[d] = pmod(c, s.M[d]) + chunk_shift[i][d] - n - org[d];
-        }
-#pragma unroll
-        for (int j = 0; j < kWPad; j++) {
-          if (FIXED)
-            rec[i].wz[j] = (WZ)__float2int_rn((float)wz[j] * (float)(1 << kWzBits));
-          else
-            rec[i].wz[j] = (WZ)wz[j];
-        }
-        rec[i].qp = a.w * s.pref;
-      }
-      __syncthreads();
-      // --- each warp: atoms that touch its patch ---
-      for (int base = 0; base < cntc; base += 32) {
-        const int i = base + lane;
-        bool rel = false;
-        if (i < cntc) {
-          const int sx = rec[i].s[0], sy = rec[i].s[1], sz = rec[i].s[2];
-          rel = sx <= px0 + 7 && sx + W - 1 >= px0 && sy <= py0 + 3 && sy + W - 1 >= py0 &&
-                sz <= ez - 1 && sz + W - 1 >= 0;
-        }
-        unsigned mask = __ballot_sync(0xffffffffu, rel);
-        while (mask) {
-          const int ia = base + __ffs(mask) - 1;
-          mask &= mask - 1;
-          const int kx = cx - rec[ia].s[0], ky = cy - rec[ia].s[1];
-          CT tf = (CT)0;
-          if ((unsigned)kx < (unsigned)W && (unsigned)ky < (unsigned)W)
-            tf = rec[ia].qp * rec[ia].w[0][kx] * rec[ia].w[1][ky];
-          T t;
-          if (FIXED)
-            t = (T)__float2int_rn((float)tf * tscale);
-          else
-            t = (T)tf;
-          WZ wz[kWPad];
-#pragma unroll
-          for (int k = 0; k < kWPad; k++) wz[k] = rec[ia].wz[k];
-          add_column_dispatch<A, T, WZ, TZ, W>(rec[ia].s[2], acc, t, wz);
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // --- write the block: every point exactly once ---
-  if (cx < ex && cy < ey) {
-    CT* col = grid + (long long)(x0 + cx) + (long long)(y0 + cy) * b.M[0];
-    const long long zs = (long long)b.M[0] * b.M[1];
-    const double unscale = FIXED ? exp2(-(double)(st + kWzBits)) : 1.0;
-#pragma unroll
-    for (int z = 0; z < TZ; z++) {
-      if (z < ez) {
-        if (FIXED)
-          col[(long long)(z0 + z) * zs] = (CT)((double)acc[z] * unscale);
-        else
-          col[(long long)(z0 + z) * zs] = (CT)acc[z];
-      }
+      for (int k = 0; k < kBasis64 / 2; k++) o[k] = make_double2(v[2 * k], v[2 * k + 1]);
     }
   }
 }
@@ -915,24 +648,19 @@ cudaError_t launch_bin_sorted(const typename Vec4<CT>::type* xyzq, int n, const 
     e = cudaMemsetAsync(w.counts, 0, sizeof(int) * nb, st);
     if (e != cudaSuccess) return e;
   }
-  // the largest |q| feeds the FP64 spread's range check only
-  unsigned* qmax = sizeof(CT) == 8 ? w.qmax_bits : nullptr;
-  if (qmax) {
-    e = cudaMemsetAsync(qmax, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
-  }
   // a grid to clear takes every SM; the atoms alone, one thread each up to that
   const int gb = w.clear ? sm_count() * 8
                          : (int)std::min<long long>(sm_count() * 8,
                                                     (n + 255) / 256 > 0 ? (n + 255) / 256 : 1);
   if (n > 0)
     k_bin_count<CT><<<gb, 256, 0, st>>>(xyzq, n, b, inv_hx, inv_hy, inv_hz, w.key, w.counts,
-                                        qmax, w.bad, w.clear, w.clear_n,
+                                        w.bad, w.clear, w.clear_n,
                                         (sizeof(CT) == 4 && w.lstart) ? w.tmp : nullptr);
   else if (w.clear)
     e = cudaMemsetAsync(w.clear, 0, sizeof(long long) * w.clear_n, st);
   if (e != cudaSuccess) return e;
-  return launch_bin_scan_place<CT>(xyzq, n, nb, w, sorted, perm, st);
+  const CT inv_h[3] = {inv_hx, inv_hy, inv_hz};
+  return launch_bin_scan_place<CT>(xyzq, n, nb, w, sorted, perm, st, b, inv_h);
 }
 
 // counts (filled) -> start offsets -> placement of the atoms: stable (in
@@ -941,7 +669,7 @@ cudaError_t launch_bin_sorted(const typename Vec4<CT>::type* xyzq, int n, const 
 template <typename CT>
 cudaError_t launch_bin_scan_place(const typename Vec4<CT>::type* xyzq, int n, int nb,
                                   BinScratch w, typename Vec4<CT>::type* sorted, int* perm,
-                                  cudaStream_t st) {
+                                  cudaStream_t st, const BinLayout& b, const CT* inv_h) {
   const int ntiles = (nb + kScanTile - 1) / kScanTile;
   if (ntiles > kScanTile) return cudaErrorInvalidValue;
   cudaError_t e;
@@ -964,26 +692,17 @@ cudaError_t launch_bin_scan_place(const typename Vec4<CT>::type* xyzq, int n, in
   k_scan_sums<<<1, kScanThreads, 0, st>>>(w.tile_sums, ntiles, w.start, nb);
   k_scan_add<<<(nb + 255) / 256, 256, 0, st>>>(w.start, nb, w.tile_sums);
   if (n > 0) {
-    if (sizeof(CT) == 4) {
+    if constexpr (sizeof(CT) == 4) {
       k_bin_place_direct<CT><<<gb, 256, 0, st>>>(xyzq, n, w.key, w.start, w.counts, sorted, perm);
     } else {
       e = cudaMemsetAsync(w.counts, 0, sizeof(int) * nb, st);
       if (e != cudaSuccess) return e;
       k_bin_place_any<<<gb, 256, 0, st>>>(n, w.key, w.start, w.counts, w.tmp);
-      k_bin_place_stable<CT><<<gb, 256, 0, st>>>(xyzq, n, w.key, w.start, w.tmp, sorted, perm);
+      const double3 ih = inv_h ? make_double3(inv_h[0], inv_h[1], inv_h[2]) : double3{};
+      k_bin_place_stable<<<gb, 256, 0, st>>>(xyzq, n, w.key, w.start, w.tmp, sorted, perm, b, ih,
+                                             w.basis);
     }
   }
-  return cudaGetLastError();
-}
-
-template <typename CT, int TZ, int W>
-static cudaError_t spread_w(const typename Vec4<CT>::type* sorted, const int* start,
-                            const unsigned* qmax_bits, const BinLayout& b, const Stencil<CT>& s,
-                            CT* grid, cudaStream_t st) {
-  const Decay<CT> dec = make_decay<CT>(s);
-  dim3 grd((b.M[0] + kTX - 1) / kTX, (b.M[1] + kTY - 1) / kTY, (b.M[2] + TZ - 1) / TZ);
-  k_spread_tiled<CT, TZ, W><<<grd, kSpreadThreads, 0, st>>>(sorted, start, qmax_bits, b, s, dec,
-                                                             grid);
   return cudaGetLastError();
 }
 
@@ -993,20 +712,6 @@ bool spread_tiled_supported(const Stencil<CT>& s) {
     if (s.nst[d] != s.nst[0]) return false;
   const int W = 2 * s.nst[0] + 1;
   return W == 9 || W == 11 || W == 13 || W == 15;
-}
-
-template <typename CT>
-cudaError_t launch_spread_tiled(const typename Vec4<CT>::type* sorted, const int* start,
-                                const unsigned* qmax_bits, const BinLayout& b,
-                                const Stencil<CT>& s, CT* grid, cudaStream_t st) {
-  constexpr int TZ = sizeof(CT) == 8 ? kTZ64 : kTZ32;
-  switch (2 * s.nst[0] + 1) {
-    case 9: return spread_w<CT, TZ, 9>(sorted, start, qmax_bits, b, s, grid, st);
-    case 11: return spread_w<CT, TZ, 11>(sorted, start, qmax_bits, b, s, grid, st);
-    case 13: return spread_w<CT, TZ, 13>(sorted, start, qmax_bits, b, s, grid, st);
-    case 15: return spread_w<CT, TZ, 15>(sorted, start, qmax_bits, b, s, grid, st);
-  }
-  return cudaErrorInvalidValue;
 }
 
 template <typename CT, int W>
@@ -1492,11 +1197,9 @@ cudaError_t launch_batch_forward_fused(const BatchFused& a, int ctas, int gather
                                              CT, CT, BinScratch, Vec4<CT>::type*, int*,         \
                                              cudaStream_t);                                     \
   template cudaError_t launch_bin_scan_place<CT>(const Vec4<CT>::type*, int, int, BinScratch,   \
-                                                 Vec4<CT>::type*, int*, cudaStream_t);          \
+                                                 Vec4<CT>::type*, int*, cudaStream_t,           \
+                                                 const BinLayout&, const CT*);                  \
   template bool spread_tiled_supported<CT>(const Stencil<CT>&);                                 \
-  template cudaError_t launch_spread_tiled<CT>(const Vec4<CT>::type*, const int*,               \
-                                               const unsigned*, const BinLayout&,               \
-                                               const Stencil<CT>&, CT*, cudaStream_t);          \
   template cudaError_t launch_gather_tiled<CT>(const Vec4<CT>::type*, const int*, const int*,   \
                                                const BinLayout&, const Stencil<CT>&, const CT*, \
                                                double, double*, double*, double*, bool,         \

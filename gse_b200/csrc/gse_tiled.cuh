@@ -14,12 +14,6 @@ namespace gse {
 // brick rows, so the mixed form bins 16 cells at a time (4x fewer bins to scan)
 constexpr int kBinX64 = 4, kBinX32 = 16;
 constexpr int kWPad = 16;           // padded stencil width (2n+1 <= 15 on the tiled path)
-constexpr int kTX = 16, kTY = 8;    // spread block columns (x, y)
-constexpr int kTZ32 = 32;           // spread block depth, mixed form (int64 accumulators)
-constexpr int kTZ64 = 24;           // spread block depth, FP64 accumulators
-constexpr int kSpreadThreads = 128; // 4 warps, each an 8 x 4 column patch
-constexpr int kSpreadChunk = 64;    // atoms staged per round
-constexpr int kMaxSeg = 4;          // periodic images of one row segment
 constexpr int kGX = 16, kGY = 16, kGZ = 8;  // gather brick (cells); kGX multiple of kBinX32
 constexpr int kGatherThreads = 256;          // >= kGY * kGZ
 constexpr int kGatherLanes = 16;             // lanes sharing one atom in the gather
@@ -45,13 +39,23 @@ struct BinLayout {
   int* flags = nullptr;
 };
 
+// What the FP64 spread needs of an atom: per axis the weight of the stencil's
+// centre point (x: times q pref) and the two ratios from which the axis' other
+// weights follow, then the wrapped x cell.  Formed once per atom here instead of
+// by every block that the atom's cube reaches (5.4 blocks of 16^3 points at n = 6).
+constexpr int kBasis64 = 10;
+struct SpreadBasis {
+  double h[3], inv_2s2, pref;
+  int nst;      // stencil half width n
+  double* out;  // [n][kBasis64] in sorted order; NULL: not wanted
+};
+
 struct BinScratch {
   int* key;        // [n]
   int* counts;     // [nbins]
   int* start;      // [nbins + 1]
   int* tile_sums;  // [ceil(nbins / 4096)]
   int* tmp;        // [n]: the FP64 stable placement's scratch; the mixed form's ranks in bin
-  unsigned* qmax_bits;  // max |q| over the atoms (float bits), written by the binning
   int* bad = nullptr;   // set to 1 when a position or charge is not finite (may be NULL)
   // mixed form: the scan's tile-local prefix [nbins] (the placement applies the tile
   // offsets and writes `start`); NULL: a three-kernel scan writes `start` directly
@@ -63,24 +67,9 @@ struct BinScratch {
   // kernel clears on the way (the mixed form's spread grid); NULL: none
   long long* clear = nullptr;
   long long clear_n = 0;
+  // FP64 form: weights' basis of the sorted atoms, for the spread that follows
+  SpreadBasis basis = {};
 };
-
-// exp(-2 h^2 / (2 sigma^2)) per axis as an unevaluated sum hi + lo in CT
-template <typename CT>
-struct Decay {
-  CT hi[3], lo[3];
-};
-template <typename CT>
-inline Decay<CT> make_decay(const Stencil<CT>& s) {
-  Decay<CT> d;
-  for (int a = 0; a < 3; a++) {
-    const double hd = (double)s.h[a];
-    const double v = std::exp(-2.0 * hd * hd * (double)s.inv_2s2);
-    d.hi[a] = (CT)v;
-    d.lo[a] = (CT)(v - (double)d.hi[a]);
-  }
-  return d;
-}
 
 inline BinLayout make_bin_layout(const int M[3], int bin_width) {
   BinLayout b;
@@ -201,15 +190,16 @@ cudaError_t launch_bin_sorted(const typename Vec4<CT>::type* xyzq, int n, const 
 template <typename CT>
 cudaError_t launch_bin_scan_place(const typename Vec4<CT>::type* xyzq, int n, int nb,
                                   BinScratch w, typename Vec4<CT>::type* sorted, int* perm,
-                                  cudaStream_t st);
+                                  cudaStream_t st, const BinLayout& b = BinLayout{},
+                                  const CT* inv_h = nullptr);
 
 template <typename CT>
 bool spread_tiled_supported(const Stencil<CT>& s);
 
-template <typename CT>
-cudaError_t launch_spread_tiled(const typename Vec4<CT>::type* sorted, const int* start,
-                                const unsigned* qmax_bits, const BinLayout& b,
-                                const Stencil<CT>& s, CT* grid, cudaStream_t st);
+// FP64 form: the whole density grid from the sorted atoms (gse_spread64.cu).
+// `basis` [n][kBasis64]: written by the binning (BinScratch::basis).
+cudaError_t launch_spread64(const double* basis, const int* start, const BinLayout& b,
+                            const Stencil<double>& s, double* grid, cudaStream_t st);
 
 // pdl: the launch follows a kernel of this library directly on `st` and may
 // overlap its end (programmatic dependent launch).
