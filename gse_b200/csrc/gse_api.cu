@@ -1736,37 +1736,23 @@ gse_status_t gse_ewald_recip(int device, void* stream, double sigma, int kcut, d
   TRY(check_xyz(device, fx, fy, fz, "force array"));
   CU(cudaSetDevice(device));
   cudaStream_t st = (cudaStream_t)stream;
-  const std::vector<EwRowHost> rows = ewald_rows(kcut);
-  long long nk = 0;
-  for (const EwRowHost& r : rows) nk += r.nk;
+  const std::vector<EwRow> rows = ewald_rows(kcut);
   EwGeom g;
   g.inv_box[0] = 1.0 / box_x;
   g.inv_box[1] = 1.0 / box_y;
   g.inv_box[2] = 1.0 / box_z;
   g.pref = 2.0 * kPi * g.inv_box[0] * g.inv_box[1] * g.inv_box[2] * ccelec;
   g.half_sigmasq = 0.5 * sigma * sigma;
-  // scratch: rows, P S(k), row energies, and staged atoms/forces
-  void* rows_d = nullptr;
-  double2* S = nullptr;
-  double* re = nullptr;
-  double4* xd = nullptr;
-  double* fd = nullptr;
+  char* buf = nullptr;
   gse_status_t status = GSE_OK;
   std::vector<double> rh(rows.size());
-  auto cleanup = [&]() {
-    cudaFree(rows_d);
-    cudaFree(S);
-    cudaFree(re);
-    cudaFree(xd);
-    cudaFree(fd);
-  };
 #define CUE(call)                                                                          \
   do {                                                                                     \
     cudaError_t _e = (call);                                                               \
     if (_e != cudaSuccess) {                                                               \
       status = fail(_e == cudaErrorMemoryAllocation ? GSE_ERR_OOM : GSE_ERR_CUDA,          \
                     "gse_ewald_recip: %s: %s", #call, cudaGetErrorString(_e));             \
-      cleanup();                                                                           \
+      cudaFree(buf);                                                                         \
       return status;                                                                       \
     }                                                                                      \
   } while (0)
@@ -1774,37 +1760,33 @@ gse_status_t gse_ewald_recip(int device, void* stream, double sigma, int kcut, d
     *energy = 0.0;
     return GSE_OK;
   }
-  CUE(cudaMalloc(&rows_d, sizeof(EwRowHost) * rows.size()));
-  CUE(cudaMalloc(&S, sizeof(double2) * nk));
-  CUE(cudaMalloc(&re, sizeof(double) * rows.size()));
+  const bool xdev = is_device_ptr(xyzq);
+  const bool fdev = want_f && is_device_ptr(fx) && is_device_ptr(fy) && is_device_ptr(fz);
+  // one allocation: the sums' scratch, then staged atoms and forces
+  const EwPlan plan = ewald_plan(n, kcut, (int)rows.size(), want_f);
+  const size_t off_x = plan.bytes, off_f = off_x + (xdev ? 0 : sizeof(double4) * (size_t)n);
+  CUE(cudaMalloc(&buf, off_f + (want_f && !fdev ? sizeof(double) * 3 * (size_t)n : 0)));
   const double4* xin = (const double4*)xyzq;
-  if (!is_device_ptr(xyzq)) {
-    CUE(cudaMalloc(&xd, sizeof(double4) * n));
-    CUE(cudaMemcpyAsync(xd, xyzq, sizeof(double4) * n, cudaMemcpyHostToDevice, st));
-    xin = xd;
+  if (!xdev) {
+    CUE(cudaMemcpyAsync(buf + off_x, xyzq, sizeof(double4) * n, cudaMemcpyHostToDevice, st));
+    xin = (const double4*)(buf + off_x);
   }
   double* f[3] = {fx, fy, fz};
-  const bool fdev = want_f && is_device_ptr(fx) && is_device_ptr(fy) && is_device_ptr(fz);
+  if (want_f && !fdev)
+    for (int k = 0; k < 3; k++) f[k] = (double*)(buf + off_f) + (size_t)k * n;
+  CUE(launch_ewald(xin, n, rows, g, plan, buf, want_f ? f[0] : nullptr, f[1], f[2], st));
+  CUE(cudaMemcpyAsync(rh.data(), buf + plan.off_energy, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost, st));
   if (want_f && !fdev) {
-    CUE(cudaMalloc(&fd, sizeof(double) * 3 * n));
-    f[0] = fd;
-    f[1] = fd + n;
-    f[2] = fd + 2 * n;
-  }
-  EwScratch w{rows_d, S, re};
-  CUE(launch_ewald(xin, n, rows, g, w, want_f ? f[0] : nullptr, f[1], f[2], st));
-  CUE(cudaMemcpyAsync(rh.data(), re, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost, st));
-  if (want_f && !fdev) {
-    CUE(cudaMemcpyAsync(fx, fd, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    CUE(cudaMemcpyAsync(fy, fd + n, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    CUE(cudaMemcpyAsync(fz, fd + 2 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+    CUE(cudaMemcpyAsync(fx, f[0], sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+    CUE(cudaMemcpyAsync(fy, f[1], sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+    CUE(cudaMemcpyAsync(fz, f[2], sizeof(double) * n, cudaMemcpyDeviceToHost, st));
   }
   CUE(cudaStreamSynchronize(st));
 #undef CUE
   double e = 0.0;
   for (double v : rh) e += v;
   *energy = e;
-  cleanup();
+  cudaFree(buf);
   return GSE_OK;
 }
 

@@ -13,21 +13,30 @@ struct EwGeom {
   double half_sigmasq;  // sigma^2 / 2
 };
 
-struct EwRowHost {
-  int ky, kz, kx0, nk;
-  long long off;
+// One row of the half space: ky, kz, and kx = kx0 .. kxm (kx0 = -kxm, or 1 on the
+// kx axis).
+struct EwRow {
+  int ky, kz, kx0, kxm;
 };
 
-struct EwScratch {
-  void* rows;          // [nrows] rows
-  double2* S;          // [number of half-space k] P(k) S(k)
-  double* row_energy;  // [nrows]
+// Sizes and scratch layout of one call (one allocation of `bytes`).
+struct EwPlan {
+  int kmax, nrows;
+  int ncols;       // columns of S: c, s of every kx, whole 8-column strips
+  int wpitch;      // the same for the force kernel, whole chunks
+  int slab, pitch; // atoms per pass, and rounded up to 64
+  int per_split, nsplit;    // atoms per split of the structure sum
+  int per_fsplit, nfsplit;  // rows per split of the force sum
+  size_t off_rows, off_energy, off_T, off_part, off_W, off_f, bytes;
 };
 
-std::vector<EwRowHost> ewald_rows(int kcut);
-cudaError_t launch_ewald(const double4* xyzq, int n, const std::vector<EwRowHost>& rows,
-                         const EwGeom& g, EwScratch w, double* fx, double* fy, double* fz,
-                         cudaStream_t st);
+// Rows of the half sphere |k| <= kcut, longest first.
+std::vector<EwRow> ewald_rows(int kcut);
+EwPlan ewald_plan(int n, int kcut, int nrows, bool forces);
+// `buf`: p.bytes of device memory; the rows' energies are left at p.off_energy.
+cudaError_t launch_ewald(const double4* xyzq, int n, const std::vector<EwRow>& rows,
+                         const EwGeom& g, const EwPlan& p, char* buf, double* fx, double* fy,
+                         double* fz, cudaStream_t st);
 
 // ---- direct (real-space) sum, gse_ewald_direct.cu ----
 
