@@ -1856,7 +1856,8 @@ gse_status_t gse_ewald_direct(int device, void* stream, double sigma, double rcu
   const size_t n_int = 2 * (size_t)n + (size_t)g.ncell * 2 + 1 + ntiles + n + 1 + ex_idx.size() +
                        (ex_start.empty() ? 0 : n + 1);
   const size_t off_d = (n_int * sizeof(int) + 31) / 32 * 32;
-  const size_t n_dbl = (size_t)g.ncell + 1 + (want_f ? 3 * (size_t)n : 0);
+  const size_t n_part = (size_t)g.ncell * ewald_direct_split(n, g);
+  const size_t n_dbl = n_part + 1 + (want_f ? 3 * (size_t)n : 0);
   const size_t off_x = (off_d + n_dbl * sizeof(double) + 31) / 32 * 32;
   const bool xdev = is_device_ptr(xyzq);
   const size_t bytes = off_x + (size_t)n * sizeof(double4) * (xdev ? 1 : 2);
@@ -1899,7 +1900,7 @@ gse_status_t gse_ewald_direct(int device, void* stream, double sigma, double rcu
   int* d_ex_start = ex_start.empty() ? nullptr : ip;
   double* dp = (double*)(buf + off_d);
   w.partials = dp;
-  double* d_energy = dp + g.ncell;
+  double* d_energy = dp + n_part;
   double* f[3] = {fx, fy, fz};
   const bool fdev = want_f && is_device_ptr(fx) && is_device_ptr(fy) && is_device_ptr(fz);
   if (want_f && !fdev)

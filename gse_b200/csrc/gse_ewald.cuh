@@ -59,11 +59,13 @@ struct EwdScratch {
   int* tmp;         // [n]
   double4* sorted;  // [n] atoms in cell order
   int* perm;        // [n] original index of each sorted atom
-  double* partials; // [ncell] energy per cell
-  unsigned* done;   // counter of finished cells
+  double* partials; // [ncell * split] energy per block
+  unsigned* done;   // counter of finished blocks
 };
 
 EwdGeom ewald_direct_geom(double sigma, double rcut, const double box[3], double ccelec);
+// Blocks per cell of the pair kernel.
+int ewald_direct_split(int n, const EwdGeom& g);
 // ex_start[n + 1] / ex_idx: the excluded partners of every atom (both
 // directions), or both NULL.  energy_out: one device double.
 cudaError_t launch_ewald_direct(const double4* xyzq, int n, const EwdGeom& g, EwdScratch w,
