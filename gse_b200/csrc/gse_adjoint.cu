@@ -156,47 +156,6 @@ __global__ void __launch_bounds__(256)
                         dy, dz);
 }
 
-// ---- batched systems: system of a sorted atom by its offset range ----
-__device__ __forceinline__ int adj_sys_of(const int* __restrict__ first, int nsys, int i) {
-  int lo = 0, hi = nsys - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (first[mid] <= i) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-__global__ void __launch_bounds__(256)
-    k_batch_adj_source(const float4* __restrict__ xyzq, const int* __restrict__ perm, int ntot,
-                       const BatchSys* __restrict__ sys, const int* __restrict__ first, int nsys,
-                       double c, const double* __restrict__ gfx, const double* __restrict__ gfy,
-                       const double* __restrict__ gfz, float* __restrict__ lambda) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int ii = gw; ii < ntot; ii += nw) {
-    const BatchSys& S = sys[adj_sys_of(first, nsys, ii)];
-    adj_source_atom<float>(xyzq[ii], perm[ii], S.sg, c, gfx, gfy, gfz, lambda + S.grid_off);
-  }
-}
-
-__global__ void __launch_bounds__(256)
-    k_batch_adj_gather(const float4* __restrict__ xyzq, const int* __restrict__ perm, int ntot,
-                       const BatchSys* __restrict__ sys, const int* __restrict__ first, int nsys,
-                       double c, const double* __restrict__ dLdE, const float* __restrict__ psi,
-                       const float* __restrict__ phi, const double* __restrict__ gfx,
-                       const double* __restrict__ gfy, const double* __restrict__ gfz,
-                       double* __restrict__ dq, double* __restrict__ dx, double* __restrict__ dy,
-                       double* __restrict__ dz) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int ii = gw; ii < ntot; ii += nw) {
-    const int si = adj_sys_of(first, nsys, ii);
-    const BatchSys& S = sys[si];
-    adj_gather_atom<float>(xyzq[ii], perm[ii], S.sp, S.sg, c, dLdE[si] * c * S.h3,
-                           psi + S.grid_off, phi + S.grid_off, gfx, gfy, gfz, dq, dx, dy, dz);
-  }
-}
-
 // ===========================================================================
 // Tiled reverse pass (mixed form)
 // ===========================================================================
@@ -210,25 +169,64 @@ __global__ void __launch_bounds__(256)
 // from the forward gather's association of the same sum only for points
 // whose distance equals the cut-off to rounding, whose weight is e^-9 of the
 // centre's.
+//
+// Bound: issue and latency.  256 uneven systems, 678,657 charges, both before and
+// after: source 1.19 -> 1.01 ms (the y tables left the registers, 112-126 -> 64, so
+// two blocks fit an SM; a block of 384 threads that spilled took 1.33 ms, two blocks
+// of 256 with the tables in registers 1.23; cotangents sorted once, 9 us; additions of
+// zero instead of a branch around each reduction, 0.88 -> 0.70 at width 13), gather
+// 1.73 -> 1.57 ms (two x offsets per packed fma in the cube rows, the 14 lane sums by
+// halves instead of 14 full butterflies, the next atom fetched ahead).
+
+constexpr int kFusedRevThreads = 512;   // the fused reverse kernel's block
+constexpr int kAdjScatterThreads = 512;  // >= kSB * kSB; 64 registers at two blocks per SM
 
 // Per-warp slots for the y tables of the reverse-pass scatter, one array for
 // every stencil width a kernel instantiates (a static array in the templated
 // function would be one per width, too much static shared memory for the
-// fused reverse kernel).
-__device__ __forceinline__ float (*adj_ytab())[3][16] {
-  __shared__ __align__(16) float t[kScatterThreads / 32][3][16];
+// fused reverse kernel).  Two neighbouring y points share a slot: e, e u of
+// both, and u^2 of both apart.
+struct AdjYTab {
+  float4 w[8];
+  float2 u2[8];
+};
+__device__ __forceinline__ AdjYTab* adj_ytab() {
+  __shared__ __align__(16) AdjYTab t[kScatterThreads / 32];
   return t;
 }
 
-template <int W>
+// The force cotangents of the sorted atoms in FP32, {Gx, Gy, Gz, |G|}: read by the
+// scatter twice per atom, in order instead of by the permutation.
+__device__ __forceinline__ float4 adj_cotangent(int o, const double* __restrict__ gfx,
+                                                const double* __restrict__ gfy,
+                                                const double* __restrict__ gfz) {
+  const float x = (float)gfx[o], y = (float)gfy[o], z = (float)gfz[o];
+  return make_float4(x, y, z, sqrtf(x * x + y * y + z * z));
+}
+
+__global__ void k_adj_sort_g(const int* __restrict__ perm, int n, const double* __restrict__ gfx,
+                             const double* __restrict__ gfy, const double* __restrict__ gfz,
+                             float4* __restrict__ gs) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    gs[i] = adj_cotangent(perm[i], gfx, gfy, gfz);
+}
+
+static cudaError_t launch_adj_sort_g(const int* perm, int n, const double* gfx, const double* gfy,
+                                     const double* gfz, float4* gs, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_adj_sort_g<<<std::min((n + 255) / 256, sm_count() * 8), 256, 0, st>>>(perm, n, gfx, gfy, gfz,
+                                                                         gs);
+  return cudaGetLastError();
+}
+
+template <int W, int NT>
 __device__ __forceinline__ void adj_scatter_brick(
-    const float4* __restrict__ sorted, const int* __restrict__ perm, const int* __restrict__ start,
-    const BinLayout& b, const Stencil<float>& s, float cA, const double* __restrict__ gfx,
-    const double* __restrict__ gfy, const double* __restrict__ gfz, int bxi, int byi, int bzi,
-    int* __restrict__ tile, long long* __restrict__ grid64) {
+    const float4* __restrict__ sorted, const float4* __restrict__ gs,
+    const int* __restrict__ start, const BinLayout& b, const Stencil<float>& s, float cA, int bxi,
+    int byi, int bzi, int* __restrict__ tile, long long* __restrict__ grid64) {
   typedef ScatterGeom<W> G;
   constexpr int n = G::n;
-  constexpr int NT = kScatterThreads, NW = NT / 32;
+  constexpr int NW = NT / 32;
   constexpr int NPASS = (W * W + 31) / 32;
   __shared__ int rng_a[kSB * kSB], rng_p[kSB * kSB];
   __shared__ int alist[kScatterList];
@@ -239,24 +237,18 @@ __device__ __forceinline__ void adj_scatter_brick(
   int total;
   const int shift = brick_prologue<W, NT>(
       start, b, x0, y0, z0, tile, rng_a, rng_p,
-      [&](int i) {
-        const int o = perm[i];
-        const float gx = (float)gfx[o], gy = (float)gfy[o], gz = (float)gfz[o];
-        return fabsf(sorted[i].w) * acA * sqrtf(gx * gx + gy * gy + gz * gz);
-      },
-      &total);
+      [&](int i) { return fabsf(sorted[i].w) * acA * gs[i].w; }, &total);
   const float tscale = exp2f((float)shift);
   // (x, z) pairs of the stencil plane each lane tests, the same for every atom
-  int psx[NPASS], psz[NPASS];
+  int psxz[NPASS];  // x | z << 8
 #pragma unroll
   for (int pass = 0; pass < NPASS; pass++) {
     const int p = pass * 32 + lane;
-    psz[pass] = p < W * W ? p / W : 0;
-    psx[pass] = p < W * W ? p - (p / W) * W : 0;
+    psxz[pass] = p < W * W ? (p - (p / W) * W) | (p / W) << 8 : 0;
   }
   // per warp: the pairs whose column meets the sphere, packed x | z << 4
   __shared__ unsigned char plist_all[NW][W * W];
-  float (*ytab)[3][16] = adj_ytab();  // e, u, u^2 along y of each warp's atom
+  AdjYTab& ytab = adj_ytab()[warp];
   unsigned char* plist = plist_all[warp];
   for (int c0 = 0; c0 < total; c0 += kScatterList) {
     brick_atom_list<NT, kSB * kSB>(rng_a, rng_p, total, c0, kScatterList, alist);
@@ -265,8 +257,8 @@ __device__ __forceinline__ void adj_scatter_brick(
     for (int q = warp; q < nc; q += NW) {
       const int ai = alist[q];
       const float4 a = sorted[ai];
-      const int o = perm[ai];
-      const float Gx = (float)gfx[o], Gy = (float)gfy[o], Gz = (float)gfz[o];
+      const float4 gv = gs[ai];
+      const float Gx = gv.x, Gy = gv.y, Gz = gv.z;
       const float pos3[3] = {a.x, a.y, a.z};
       const int org[3] = {x0, y0, z0};
       int loc[3];
@@ -281,56 +273,30 @@ __device__ __forceinline__ void adj_scatter_brick(
         u2l[d] = u2;
         el[d] = (lane < W) ? expf(mul_rn(-u2, s.inv_2s2)) : 0.f;
       }
-      // the y tables every lane needs, through the warp's shared slots and
-      // 16-byte broadcast loads rather than 39 shuffles (as in the spread)
-      float ey[W], eyuy[W], uy2[W];
-      {
-        __syncwarp();  // the warp's previous atom has read its tables
-        if (lane < 16) {
-          ytab[warp][0][lane] = el[1];
-          ytab[warp][1][lane] = ul[1];
-          ytab[warp][2][lane] = u2l[1];
-        }
-        __syncwarp();
-        float uy[W];
-        const float4* v0 = reinterpret_cast<const float4*>(ytab[warp][0]);
-        const float4* v1 = reinterpret_cast<const float4*>(ytab[warp][1]);
-        const float4* v2 = reinterpret_cast<const float4*>(ytab[warp][2]);
-#pragma unroll
-        for (int q4 = 0; q4 < (W + 3) / 4; q4++) {
-          const float4 a = v0[q4], b = v1[q4], c = v2[q4];
-          const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w},
-                      cv[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (4 * q4 + j < W) {
-              ey[4 * q4 + j] = av[j];
-              uy[4 * q4 + j] = bv[j];
-              uy2[4 * q4 + j] = cv[j];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < W; k++) eyuy[k] = ey[k] * uy[k];
+      // the y tables every lane needs, through the warp's shared slots; read again
+      // for every pass by broadcast loads (in registers, 3 W of them, they cost half
+      // of the warps an SM can hold)
+      __syncwarp();  // the warp's previous atom has read its tables
+      if (lane < 16) {
+        float* w = reinterpret_cast<float*>(&ytab.w[lane >> 1]) + (lane & 1);
+        w[0] = el[1];
+        w[2] = el[1] * ul[1];
+        reinterpret_cast<float*>(ytab.u2)[lane] = lane < W ? u2l[1] : __int_as_float(0x7f800000);
       }
-      // the same weights in pairs of y points for the packed fma
-      unsigned long long ey2[W / 2], eyuy2[W / 2], magic2;
-#pragma unroll
-      for (int k = 0; k + 1 < W; k += 2) {
-        asm("mov.b64 %0, {%1, %2};" : "=l"(ey2[k / 2]) : "f"(ey[k]), "f"(ey[k + 1]));
-        asm("mov.b64 %0, {%1, %2};" : "=l"(eyuy2[k / 2]) : "f"(eyuy[k]), "f"(eyuy[k + 1]));
-      }
+      __syncwarp();
+      unsigned long long magic2;
       asm("mov.b64 %0, {%1, %1};" : "=l"(magic2) : "f"(12582912.0f));
       // compact the (x, z) pairs with u_x^2 + u_z^2 < rcut^2: every point of
       // the other columns lies outside the sphere
       int npair = 0;
 #pragma unroll
       for (int pass = 0; pass < NPASS; pass++) {
-        const float ux2 = __shfl_sync(0xffffffffu, u2l[0], psx[pass]);
-        const float uz2 = __shfl_sync(0xffffffffu, u2l[2], psz[pass]);
+        const float ux2 = __shfl_sync(0xffffffffu, u2l[0], psxz[pass] & 15);
+        const float uz2 = __shfl_sync(0xffffffffu, u2l[2], psxz[pass] >> 8);
         const bool ne = pass * 32 + lane < W * W && ux2 + uz2 < s.rcut2;
         const unsigned m = __ballot_sync(0xffffffffu, ne);
         if (ne) plist[npair + __popc(m & ((1u << lane) - 1u))] =
-            (unsigned char)(psx[pass] | (psz[pass] << 4));
+            (unsigned char)((psxz[pass] & 15) | (psxz[pass] >> 8 << 4));
         npair += __popc(m);
       }
       __syncwarp();
@@ -355,21 +321,24 @@ __device__ __forceinline__ void adj_scatter_brick(
           asm("mov.b64 %0, {%1, %1};" : "=l"(t1p) : "f"(t1));
           asm("mov.b64 %0, {%1, %1};" : "=l"(t2p) : "f"(t2));
 #pragma unroll
-          for (int k = 0; k + 1 < W; k += 2) {
+          for (int k = 0; k < (W + 1) / 2; k++) {
             // |t1 e_y + t2 e_y u_y| < 2^22: both roundings stay at unit spacing;
-            // two y points per packed fma, each half rounded as fmaf rounds
-            unsigned long long r2;
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r2) : "l"(t2p), "l"(eyuy2[k / 2]), "l"(magic2));
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(r2) : "l"(t1p), "l"(ey2[k / 2]));
+            // two y points per packed fma, each half rounded as fmaf rounds; the
+            // point past the last fails its test
+            const float4 w4 = ytab.w[k];
+            const float2 v2 = ytab.u2[k];
+            unsigned long long e2, eu2, r2;
+            asm("mov.b64 %0, {%1, %2};" : "=l"(e2) : "f"(w4.x), "f"(w4.y));
+            asm("mov.b64 %0, {%1, %2};" : "=l"(eu2) : "f"(w4.z), "f"(w4.w));
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r2) : "l"(t2p), "l"(eu2), "l"(magic2));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(r2) : "l"(t1p), "l"(e2));
             unsigned lo, hi;
             asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(r2));
-            if (uy2[k] < rem) atomicAdd(cell + k * G::RP, (int)lo - 0x4B400000);
-            if (uy2[k + 1] < rem) atomicAdd(cell + (k + 1) * G::RP, (int)hi - 0x4B400000);
-          }
-          if (uy2[W - 1] < rem) {
-            const int v = __float_as_int(fmaf(t1, ey[W - 1], fmaf(t2, eyuy[W - 1], 12582912.0f))) -
-                          0x4B400000;
-            atomicAdd(cell + (W - 1) * G::RP, v);
+            // a point outside the sphere adds zero: a reduction costs the same for one
+            // lane as for all, a branch around each costs more
+            atomicAdd(cell + 2 * k * G::RP, v2.x < rem ? (int)lo - 0x4B400000 : 0);
+            if (2 * k + 1 < W)
+              atomicAdd(cell + (2 * k + 1) * G::RP, v2.y < rem ? (int)hi - 0x4B400000 : 0);
           }
         }
       }
@@ -416,6 +385,7 @@ __device__ __forceinline__ void adj_gather_brick(
   float* tphi = tpsi + TZ * ZP;                      // [TZ][ZP]
   float* tabs = tphi + TZ * ZP;                      // [NW][APW][axis][u, u^2, e][kWPad]
   int* rowl = (int*)(tabs + NW * APW * 9 * kWPad);   // [NW][APW][W*W]
+  static_assert(GL == 32, "a warp per atom");
   __shared__ int rng_a[NR], rng_p[NR + 1];
   __shared__ int alist[kGatherList];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -465,11 +435,27 @@ __device__ __forceinline__ void adj_gather_brick(
     brick_atom_list<NT, NR>(rng_a, rng_p, natoms, c0, kGatherList, alist);
     __syncthreads();
     const int nc = min(kGatherList, natoms - c0);
-    for (int q0 = APW * warp; q0 < nc; q0 += APW * NW) {
-      const int q = q0 + grp;
-      const bool valid = q < nc;
-      const int ai = alist[valid ? q : q0];
-      const float4 a = sorted[ai];
+    // the next atom's record and output slot are loaded one iteration ahead, this
+    // atom's cotangents (by the slot) ahead of its sums, which need them last
+    float4 a_n;
+    int o_n = 0;
+    if (warp < nc) {
+      a_n = sorted[alist[warp]];
+      o_n = perm[alist[warp]];
+    }
+    for (int q = warp; q < nc; q += NW) {
+      const float4 a = a_n;
+      const int o = o_n;
+      double G[3] = {0.0, 0.0, 0.0};
+      if (lane < 4 && gfx) {
+        G[0] = gfx[o];
+        G[1] = gfy[o];
+        G[2] = gfz[o];
+      }
+      if (q + NW < nc) {
+        a_n = sorted[alist[q + NW]];
+        o_n = perm[alist[q + NW]];
+      }
       const float pos3[3] = {a.x, a.y, a.z};
       const int org[3] = {x0, y0, z0};
       int loc[3];
@@ -486,30 +472,40 @@ __device__ __forceinline__ void adj_gather_brick(
         }
       }
       __syncwarp();
-      unsigned long long w2[W];  // (e_x, e_x u_x) per x offset
+      // (e_x, e_x u_x) per x offset, as scalars and in pairs of offsets
+      float ex[W], eux[W];
+      unsigned long long e2[W / 2], eu2p[W / 2];
 #pragma unroll
       for (int k = 0; k < W; k++) {
-        const float e = tb[(0 * 3 + 2) * kWPad + k];
-        const float eu = e * tb[(0 * 3 + 0) * kWPad + k];
-        asm("mov.b64 %0, {%1, %2};" : "=l"(w2[k]) : "f"(e), "f"(eu));
+        ex[k] = tb[(0 * 3 + 2) * kWPad + k];
+        eux[k] = ex[k] * tb[(0 * 3 + 0) * kWPad + k];
       }
-      // cube rows of Psi: P = sum e Psi, V = sum e Psi u (a lane's rows summed in
-      // FP32, the lanes' sums in FP64 below)
+#pragma unroll
+      for (int k = 0; k < W / 2; k++) {
+        asm("mov.b64 %0, {%1, %2};" : "=l"(e2[k]) : "f"(ex[2 * k]), "f"(ex[2 * k + 1]));
+        asm("mov.b64 %0, {%1, %2};" : "=l"(eu2p[k]) : "f"(eux[2 * k]), "f"(eux[2 * k + 1]));
+      }
+      // cube rows of Psi: P = sum e Psi, V = sum e Psi u, two offsets per packed fma
+      // (a lane's rows summed in FP32, the lanes' sums in FP64 below)
       float P = 0.f, Vx = 0.f, Vy = 0.f, Vz = 0.f;
 #pragma unroll
       for (int g = 0; g < NG; g++) {
         if (g * GL + gl < W * W) {
           const int jy = gjy[g], jz = gjz[g];
           const float* row = tpsi + (loc[2] + jz) * ZP + (loc[1] + jy) * TP + loc[0];
-          unsigned long long acc = 0ull;
+          unsigned long long s0 = 0ull, s1 = 0ull;
 #pragma unroll
-          for (int k = 0; k < W; k++) {
+          for (int k = 0; k < W / 2; k++) {
             unsigned long long p2;
-            asm("mov.b64 %0, {%1, %1};" : "=l"(p2) : "f"(row[k]));
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(w2[k]), "l"(p2));
+            asm("mov.b64 %0, {%1, %2};" : "=l"(p2) : "f"(row[2 * k]), "f"(row[2 * k + 1]));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s0) : "l"(e2[k]), "l"(p2));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(s1) : "l"(eu2p[k]), "l"(p2));
           }
-          float r0, r1;
-          asm("mov.b64 {%0, %1}, %2;" : "=f"(r0), "=f"(r1) : "l"(acc));
+          float r0, r0b, r1, r1b;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(r0), "=f"(r0b) : "l"(s0));
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(r1), "=f"(r1b) : "l"(s1));
+          r0 = fmaf(ex[W - 1], row[W - 1], r0 + r0b);
+          r1 = fmaf(eux[W - 1], row[W - 1], r1 + r1b);
           const float w = tb[(1 * 3 + 2) * kWPad + jy] * tb[(2 * 3 + 2) * kWPad + jz];
           const float a0 = w * r0;
           P += a0;
@@ -532,11 +528,10 @@ __device__ __forceinline__ void adj_gather_brick(
         nrow += __popc(m);
       }
       __syncwarp();
-      float dx2[W], ex[W], eux[W], eu2[W];
+      float dx2[W], eu2[W];
 #pragma unroll
       for (int k = 0; k < W; k++) {
         dx2[k] = tb[(0 * 3 + 1) * kWPad + k];
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(ex[k]), "=f"(eux[k]) : "l"(w2[k]));
         eu2[k] = ex[k] * dx2[k];
       }
       float T0 = 0, T1x = 0, T1y = 0, T1z = 0;
@@ -583,23 +578,37 @@ __device__ __forceinline__ void adj_gather_brick(
         Myz += a0 * uy * uz;
         Mzz += a0 * uz2;
       }
-      double acc14[14] = {P, Vx, Vy, Vz, T0, T1x, T1y, T1z, Mxx, Mxy, Mxz, Myy, Myz, Mzz};
+      // the lanes' sums in FP64: at each step a lane keeps half of its values and
+      // hands the other half to its partner (the butterfly's sums, at a third of its
+      // shuffles); lane 2 i then holds value i, and the first four lanes form one
+      // output each
+      double v[16] = {P, Vx, Vy, Vz, T0, T1x, T1y, T1z, Mxx, Mxy, Mxz, Myy, Myz, Mzz, 0.0, 0.0};
 #pragma unroll
-      for (int o = GL / 2; o > 0; o >>= 1)
+      for (int h = 8; h > 0; h >>= 1) {
+        const bool up = lane & (2 * h);
 #pragma unroll
-        for (int v = 0; v < 14; v++) acc14[v] += __shfl_xor_sync(0xffffffffu, acc14[v], o);
-      if (gl == 0 && valid) {
-        const int o = perm[ai];
-        const double q = (double)a.w;
-        const double Gx = gfx ? gfx[o] : 0.0, Gy = gfy ? gfy[o] : 0.0, Gz = gfz ? gfz[o] : 0.0;
-        const double T2x = acc14[8] * Gx + acc14[9] * Gy + acc14[10] * Gz;
-        const double T2y = acc14[9] * Gx + acc14[11] * Gy + acc14[12] * Gz;
-        const double T2z = acc14[10] * Gx + acc14[12] * Gy + acc14[13] * Gz;
-        const double vs = -pref_sp * inv_s2;  // (r - x) = -u
-        dq[o] = pref_sp * acc14[0] + cA * (Gx * acc14[5] + Gy * acc14[6] + Gz * acc14[7]);
-        dx[o] = q * vs * acc14[1] + cA * q * (Gx * acc14[4] - T2x * inv_s2);
-        dy[o] = q * vs * acc14[2] + cA * q * (Gy * acc14[4] - T2y * inv_s2);
-        dz[o] = q * vs * acc14[3] + cA * q * (Gz * acc14[4] - T2z * inv_s2);
+        for (int i = 0; i < h; i++) {
+          const double give = up ? v[i] : v[i + h];
+          v[i] = (up ? v[i + h] : v[i]) + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+        }
+      }
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      double* m = reinterpret_cast<double*>(tb);  // the atom's tables are used up
+      __syncwarp();
+      if (!(lane & 1)) m[lane >> 1] = v[0];
+      __syncwarp();
+      if (lane < 4) {
+        const double q64 = (double)a.w;
+        // lane 0: dL/dq from T1; lane 1 + d: dL/dx_d from row d of M
+        const int i0 = lane == 0 ? 5 : 7 + lane, i1 = lane == 0 ? 6 : lane == 1 ? 9 : 9 + lane,
+                  i2 = lane == 0 ? 7 : lane == 1 ? 10 : 10 + lane;
+        const double t = m[i0] * G[0] + m[i1] * G[1] + m[i2] * G[2];
+        const double Gd = lane == 1 ? G[0] : lane == 2 ? G[1] : G[2];
+        double* out = lane == 0 ? dq : lane == 1 ? dx : lane == 2 ? dy : dz;
+        // (r - x) = -u
+        out[o] = lane == 0 ? pref_sp * m[0] + cA * t
+                           : -q64 * pref_sp * inv_s2 * m[lane] +
+                                 cA * q64 * (Gd * m[4] - t * inv_s2);
       }
       __syncwarp();
     }
@@ -608,14 +617,13 @@ __device__ __forceinline__ void adj_gather_brick(
 }
 
 template <int W>
-__global__ void __launch_bounds__(kScatterThreads)
-    k_adj_scatter(const float4* __restrict__ sorted, const int* __restrict__ perm,
+__global__ void __launch_bounds__(kAdjScatterThreads, 2)
+    k_adj_scatter(const float4* __restrict__ sorted, const float4* __restrict__ gs,
                   const int* __restrict__ start, BinLayout b, Stencil<float> s, float cA,
-                  const double* __restrict__ gfx, const double* __restrict__ gfy,
-                  const double* __restrict__ gfz, long long* __restrict__ grid64) {
+                  long long* __restrict__ grid64) {
   extern __shared__ int atile[];
-  adj_scatter_brick<W>(sorted, perm, start, b, s, cA, gfx, gfy, gfz, blockIdx.x, blockIdx.y,
-                       blockIdx.z, atile, grid64);
+  adj_scatter_brick<W, kAdjScatterThreads>(sorted, gs, start, b, s, cA, blockIdx.x, blockIdx.y,
+                                           blockIdx.z, atile, grid64);
 }
 
 template <int W>
@@ -633,19 +641,18 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
 }
 
 template <int W>
-__global__ void __launch_bounds__(kScatterThreads)
-    k_batch_adj_scatter(const float4* __restrict__ sorted, const int* __restrict__ perm,
+__global__ void __launch_bounds__(kAdjScatterThreads, 2)
+    k_batch_adj_scatter(const float4* __restrict__ sorted, const float4* __restrict__ gs,
                         const int* __restrict__ start, const BatchSys* __restrict__ sys,
                         const BatchItem* __restrict__ items, int nitems, double c,
-                        const double* __restrict__ gfx, const double* __restrict__ gfy,
-                        const double* __restrict__ gfz, long long* __restrict__ grid64) {
+                        long long* __restrict__ grid64) {
   extern __shared__ int atile[];
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const BatchItem item = items[it];
     const BatchSys& S = sys[item.sys];
     const float cA = (float)(c * (double)S.sg.pref);
-    adj_scatter_brick<W>(sorted, perm, start + S.bin_off, S.b, S.sg, cA, gfx, gfy, gfz, item.bx,
-                         item.by, item.bz, atile, grid64 + S.grid_off);
+    adj_scatter_brick<W, kAdjScatterThreads>(sorted, gs, start + S.bin_off, S.b, S.sg, cA, item.bx,
+                                             item.by, item.bz, atile, grid64 + S.grid_off);
     __syncthreads();
   }
 }
@@ -686,10 +693,9 @@ cudaError_t set_smem_once(K kernel, size_t bytes, std::atomic<bool>* done) {
 }
 
 template <int W>
-cudaError_t adj_scatter_w(const float4* sorted, const int* perm, const int* start,
-                          const BinLayout& b, const Stencil<float>& s, double c, const double* gfx,
-                          const double* gfy, const double* gfz, long long* grid64, float* lambda,
-                          cudaStream_t st) {
+cudaError_t adj_scatter_w(const float4* sorted, const float4* gs, const int* start,
+                          const BinLayout& b, const Stencil<float>& s, double c,
+                          long long* grid64, float* lambda, cudaStream_t st) {
   static std::atomic<bool> done[64];
   const size_t smem = sizeof(int) * ScatterGeom<W>::words;
   cudaError_t e = set_smem_once(k_adj_scatter<W>, smem, done);
@@ -698,9 +704,8 @@ cudaError_t adj_scatter_w(const float4* sorted, const int* perm, const int* star
   e = cudaMemsetAsync(grid64, 0, sizeof(long long) * size, st);
   if (e != cudaSuccess) return e;
   const dim3 grd((b.M[0] + kSB - 1) / kSB, (b.M[1] + kSB - 1) / kSB, (b.M[2] + kSB - 1) / kSB);
-  k_adj_scatter<W><<<grd, kScatterThreads, smem, st>>>(sorted, perm, start, b, s,
-                                                       (float)(c * (double)s.pref), gfx, gfy, gfz,
-                                                       grid64);
+  k_adj_scatter<W><<<grd, kAdjScatterThreads, smem, st>>>(sorted, gs, start, b, s,
+                                                          (float)(c * (double)s.pref), grid64);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_grid64_to_real(grid64, size, lambda, st);
@@ -723,15 +728,17 @@ cudaError_t adj_gather_w(const float4* sorted, const int* perm, const int* start
 }
 }  // namespace
 
-cudaError_t launch_adj_scatter(const float4* sorted, const int* perm, const int* start,
+cudaError_t launch_adj_scatter(const float4* sorted, const int* perm, int n, const int* start,
                                const BinLayout& b, const Stencil<float>& sg, double c,
                                const double* gfx, const double* gfy, const double* gfz,
-                               long long* grid64, float* lambda, cudaStream_t st) {
+                               float4* gs, long long* grid64, float* lambda, cudaStream_t st) {
+  const cudaError_t e = launch_adj_sort_g(perm, n, gfx, gfy, gfz, gs, st);
+  if (e != cudaSuccess) return e;
   switch (2 * sg.nst[0] + 1) {
-    case 9: return adj_scatter_w<9>(sorted, perm, start, b, sg, c, gfx, gfy, gfz, grid64, lambda, st);
-    case 11: return adj_scatter_w<11>(sorted, perm, start, b, sg, c, gfx, gfy, gfz, grid64, lambda, st);
-    case 13: return adj_scatter_w<13>(sorted, perm, start, b, sg, c, gfx, gfy, gfz, grid64, lambda, st);
-    case 15: return adj_scatter_w<15>(sorted, perm, start, b, sg, c, gfx, gfy, gfz, grid64, lambda, st);
+    case 9: return adj_scatter_w<9>(sorted, gs, start, b, sg, c, grid64, lambda, st);
+    case 11: return adj_scatter_w<11>(sorted, gs, start, b, sg, c, grid64, lambda, st);
+    case 13: return adj_scatter_w<13>(sorted, gs, start, b, sg, c, grid64, lambda, st);
+    case 15: return adj_scatter_w<15>(sorted, gs, start, b, sg, c, grid64, lambda, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -751,13 +758,15 @@ cudaError_t launch_adj_gather_tiled(const float4* sorted, const int* perm, const
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_batch_adj_scatter(const float4* sorted, const int* perm, const int* start,
-                                     const BatchSys* sys, const BatchItem* items,
-                                     const BatchSeg* segs, int nseg, int ctas, double c,
-                                     const double* gfx, const double* gfy, const double* gfz,
-                                     long long* grid64, long long gsize, float* lambda,
-                                     cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(grid64, 0, sizeof(long long) * gsize, st);
+cudaError_t launch_batch_adj_scatter(const float4* sorted, const int* perm, int ntot,
+                                     const int* start, const BatchSys* sys,
+                                     const BatchItem* items, const BatchSeg* segs, int nseg,
+                                     int ctas, double c, const double* gfx, const double* gfy,
+                                     const double* gfz, float4* gs, long long* grid64,
+                                     long long gsize, float* lambda, cudaStream_t st) {
+  cudaError_t e = launch_adj_sort_g(perm, ntot, gfx, gfy, gfz, gs, st);
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(grid64, 0, sizeof(long long) * gsize, st);
   if (e != cudaSuccess) return e;
   for (int k = 0; k < nseg; k++) {
     const BatchItem* it = items + segs[k].first;
@@ -769,9 +778,8 @@ cudaError_t launch_batch_adj_scatter(const float4* sorted, const int* perm, cons
     const size_t smem = sizeof(int) * ScatterGeom<WW>::words;                                \
     e = set_smem_once(k_batch_adj_scatter<WW>, smem, done);                                  \
     if (e == cudaSuccess)                                                                    \
-      k_batch_adj_scatter<WW><<<cnt, kScatterThreads, smem, st>>>(sorted, perm, start, sys,  \
-                                                                  it, ni, c, gfx, gfy, gfz,  \
-                                                                  grid64);                   \
+      k_batch_adj_scatter<WW><<<cnt, kAdjScatterThreads, smem, st>>>(                   \
+          sorted, gs, start, sys, it, ni, c, grid64);                                        \
     break;                                                                                   \
   }
     switch (segs[k].W) {
@@ -834,7 +842,6 @@ cudaError_t launch_batch_adj_gather_tiled(const float4* sorted, const int* perm,
 // reverse-pass gather.  Reads the forward pass's sorted atoms, bins and
 // potential.
 // ---------------------------------------------------------------------------
-constexpr int kFusedRevThreads = 512;
 static_assert(kFusedRevThreads == kScatterThreads, "the fused kernel runs the scatter bricks");
 
 constexpr size_t cmax_rev(size_t a, size_t b) { return a > b ? a : b; }
@@ -855,6 +862,8 @@ __global__ void __launch_bounds__(kFusedRevThreads, 1) k_batch_reverse_fused(Bat
   const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long gstride = (long long)gridDim.x * blockDim.x;
   for (long long i = gtid; i < a.gtot; i += gstride) a.g64[i] = 0;
+  for (long long i = gtid; i < a.ntot; i += gstride)
+    a.gs[i] = adj_cotangent(a.perm[i], a.gfx, a.gfy, a.gfz);
   if (gtid < 2) a.qctr[2 + gtid] = 0;
   cg::this_grid().sync();
   for (int it = fused_next_item(&a.qctr[2]); it < a.nscat; it = fused_next_item(&a.qctr[2])) {
@@ -865,14 +874,14 @@ __global__ void __launch_bounds__(kFusedRevThreads, 1) k_batch_reverse_fused(Bat
     int* tile = reinterpret_cast<int*>(fsm);
     const float cA = (float)(a.ccelec * (double)S.sg.pref);
     switch (S.W) {
-      case 9: adj_scatter_brick<9>(a.sorted, a.perm, st, S.b, S.sg, cA, a.gfx, a.gfy, a.gfz,
-                                   item.bx, item.by, item.bz, tile, g); break;
-      case 11: adj_scatter_brick<11>(a.sorted, a.perm, st, S.b, S.sg, cA, a.gfx, a.gfy, a.gfz,
-                                     item.bx, item.by, item.bz, tile, g); break;
-      case 13: adj_scatter_brick<13>(a.sorted, a.perm, st, S.b, S.sg, cA, a.gfx, a.gfy, a.gfz,
-                                     item.bx, item.by, item.bz, tile, g); break;
-      default: adj_scatter_brick<15>(a.sorted, a.perm, st, S.b, S.sg, cA, a.gfx, a.gfy, a.gfz,
-                                     item.bx, item.by, item.bz, tile, g); break;
+      case 9: adj_scatter_brick<9, kFusedRevThreads>(
+          a.sorted, a.gs, st, S.b, S.sg, cA, item.bx, item.by, item.bz, tile, g); break;
+      case 11: adj_scatter_brick<11, kFusedRevThreads>(
+          a.sorted, a.gs, st, S.b, S.sg, cA, item.bx, item.by, item.bz, tile, g); break;
+      case 13: adj_scatter_brick<13, kFusedRevThreads>(
+          a.sorted, a.gs, st, S.b, S.sg, cA, item.bx, item.by, item.bz, tile, g); break;
+      default: adj_scatter_brick<15, kFusedRevThreads>(
+          a.sorted, a.gs, st, S.b, S.sg, cA, item.bx, item.by, item.bz, tile, g); break;
     }
     __syncthreads();
   }
@@ -945,28 +954,6 @@ cudaError_t launch_batch_reverse_fused(const BatchFused& a, int ctas, cudaStream
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k_batch_reverse_fused, a);
-}
-
-cudaError_t launch_batch_adj_source(const float4* xyzq, const int* perm, int ntot,
-                                    const BatchSys* sys, const int* first, int nsys, double c,
-                                    const double* gfx, const double* gfy, const double* gfz,
-                                    float* lambda, cudaStream_t st) {
-  if (ntot <= 0) return cudaSuccess;
-  k_batch_adj_source<<<sm_count() * 16, 256, 0, st>>>(xyzq, perm, ntot, sys, first, nsys, c, gfx, gfy,
-                                               gfz, lambda);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_batch_adj_gather(const float4* xyzq, const int* perm, int ntot,
-                                    const BatchSys* sys, const int* first, int nsys, double c,
-                                    const double* dLdE, const float* psi, const float* phi,
-                                    const double* gfx, const double* gfy, const double* gfz,
-                                    double* dq, double* dx, double* dy, double* dz,
-                                    cudaStream_t st) {
-  if (ntot <= 0) return cudaSuccess;
-  k_batch_adj_gather<<<sm_count() * 16, 256, 0, st>>>(xyzq, perm, ntot, sys, first, nsys, c, dLdE, psi,
-                                               phi, gfx, gfy, gfz, dq, dx, dy, dz);
-  return cudaGetLastError();
 }
 
 template <typename CT>

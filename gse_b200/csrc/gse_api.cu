@@ -1623,12 +1623,12 @@ gse_status_t gse_adjoint(gse_context_t* c, int n, const void* xyzq, double dLdE,
     cudaFree(c->d_adj);
     c->d_adj = nullptr;
     c->adj_cap = 0;
-    CU(cudaMalloc(&c->d_adj, 7 * c->atom_cap * sizeof(double)));
+    CU(cudaMalloc(&c->d_adj, 9 * c->atom_cap * sizeof(double)));
     c->adj_cap = c->atom_cap;
   }
   const size_t cap = c->adj_cap;
   double* g = c->d_adj;           // upstream dL/dF (3 x cap)
-  double* o = c->d_adj + 3 * cap; // dq, dx, dy, dz (4 x cap)
+  double* o = c->d_adj + 3 * cap; // dq, dx, dy, dz (4 x cap), then float4 scratch
   const double* gd[3] = {nullptr, nullptr, nullptr};
   if (have_g) {
     const double* gin[3] = {gfx, gfy, gfz};
@@ -1667,10 +1667,10 @@ gse_status_t gse_adjoint(gse_context_t* c, int n, const void* xyzq, double dLdE,
       !c->fp64 && tiled_ok<float>(c, stencil_of<float>(c, box.v, c->sigma1, c->rcut1, true, false));
   if (tiled_mixed) {
     const Stencil<float> sg = stencil_of<float>(c, box.v, c->sigma1, c->rcut1, true, false);
-    c->launches += 2;
-    CU(launch_adj_scatter((const float4*)c->d_sorted, c->d_perm, c->d_bstart, c->bl, sg,
-                          c->p.ccelec, gd[0], gd[1], gd[2], c->d_fixed, (float*)c->d_rho,
-                          c->stream));
+    c->launches += 3;
+    CU(launch_adj_scatter((const float4*)c->d_sorted, c->d_perm, n, c->d_bstart, c->bl, sg,
+                          c->p.ccelec, gd[0], gd[1], gd[2], (float4*)(c->d_adj + 7 * cap),
+                          c->d_fixed, (float*)c->d_rho, c->stream));
   } else {
   CU(cudaMemsetAsync(c->d_rho, 0, c->size * c->ct, c->stream));
   c->launches += 3;

@@ -83,6 +83,7 @@ struct gse_batch {
   double* d_forces = nullptr;  // 3 x ntot
   double* d_dLdE = nullptr;    // nsys
   double* d_gin = nullptr;     // 3 x ntot
+  float4* d_gs = nullptr;      // ntot: sorted cotangents (scratch)
   double* d_gout = nullptr;    // 4 x ntot
   int scat_ctas = 0, gath_ctas = 0, agath_ctas = 0;
   bool largest_first = false;
@@ -243,6 +244,7 @@ BatchFused fused_args(const gse_batch_t* b) {
   a.dLdE = b->d_dLdE;
   const long long nt = b->ntot;
   a.gfx = b->d_gin;
+  a.gs = b->d_gs;
   a.gfy = b->d_gin + nt;
   a.gfz = b->d_gin + 2 * nt;
   a.dq = b->d_gout;
@@ -286,10 +288,11 @@ gse_status_t run_adjoint(gse_batch_t* b) {
     return GSE_OK;
   }
   const long long nt = b->ntot;
-  BCU(launch_batch_adj_scatter(b->d_sorted, b->d_perm, b->d_start, b->d_sys, b->d_scat,
+  BCU(launch_batch_adj_scatter(b->d_sorted, b->d_perm, b->ntot, b->d_start, b->d_sys, b->d_scat,
                                b->scat_seg.data(), (int)b->scat_seg.size(), b->scat_ctas,
                                b->p.ccelec, b->d_gin,
-                               b->d_gin + nt, b->d_gin + 2 * nt, b->d_g64, b->gtot, b->d_lam, st));
+                               b->d_gin + nt, b->d_gin + 2 * nt, b->d_gs, b->d_g64, b->gtot, b->d_lam,
+                               st));
   for (const SizeClass& c : b->cls)
     BFFT(cufftExecR2C(c.pf, (cufftReal*)(b->d_lam + c.goff), (cufftComplex*)(b->d_rhok + c.koff)));
   BCU(launch_batch_green(b->d_rhok, b->d_gtab, b->ktot, b->d_sys, b->d_kfirst, b->d_ksys, b->nsys,
@@ -469,6 +472,7 @@ gse_status_t gse_batch_create(const gse_params_t* common, int nsys, const gse_sy
   BCUC(cudaMalloc(&b->d_dLdE, sizeof(double) * nsys));
   BCUC(cudaMalloc(&b->d_forces, sizeof(double) * 3 * na));
   BCUC(cudaMalloc(&b->d_gin, sizeof(double) * 3 * na));
+  BCUC(cudaMalloc(&b->d_gs, sizeof(float4) * na));
   BCUC(cudaMalloc(&b->d_gout, sizeof(double) * 4 * na));
   BCUC(cudaMemset(b->d_gin, 0, sizeof(double) * 3 * na));
   BCUC(cudaMemset(b->d_dLdE, 0, sizeof(double) * nsys));
@@ -558,7 +562,7 @@ gse_status_t gse_batch_destroy(gse_batch_t* b) {
                   b->d_sys, b->d_first, b->d_kfirst, b->d_ksys, b->d_scat, b->d_gath, b->d_agath,
                   b->d_xyzq, b->d_sorted, b->d_perm, b->d_key, b->d_tmp, b->d_counts,
                   b->d_start, b->d_tiles, b->d_g64, b->d_rho, b->d_phi, b->d_lam,
-                  b->d_rhok, b->d_gtab, b->d_energy, b->d_dLdE, b->d_forces, b->d_gin,
+                  b->d_rhok, b->d_gtab, b->d_energy, b->d_dLdE, b->d_forces, b->d_gin, b->d_gs,
                   b->d_gout};
   for (void* q : ptrs) cudaFree(q);
   delete b;

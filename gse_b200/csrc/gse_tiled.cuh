@@ -142,6 +142,7 @@ struct BatchFused {
   double *fx, *fy, *fz;     // forces [ntot]
   const double* dLdE;       // reverse pass inputs
   const double *gfx, *gfy, *gfz;
+  float4* gs;               // [ntot] the sorted atoms' cotangents (scratch)
   double *dq, *dx, *dy, *dz;  // reverse pass outputs
   int* qctr;                // [4] work-item counters: spread, gather, adjoint source,
                             // reverse-pass gather (each kernel zeroes its own first)
