@@ -407,27 +407,94 @@ __device__ __forceinline__ void row_sums(const CT* row, const CT (&dx2)[W], cons
 
 // Shared memory of the gather for calculation type CT and stencil width W:
 // the potential tile [TZ][ZP] (rows of pitch TP), per-atom weight tables and
-// per-atom row lists.
-template <typename CT, int W, int NT = kGatherThreads, int GL = kGatherLanes>
+// the list of stencil rows.
+template <typename CT, int W, int NT = kGatherThreads, int GL = kGatherLanes, int GY = kGY,
+          int GZ = kGZ>
 struct GatherGeom {
   static constexpr int n = (W - 1) / 2;
-  static constexpr int TX = kGX + 2 * n, TY = kGY + 2 * n, TZ = kGZ + 2 * n;
+  static constexpr int TX = kGX + 2 * n, TY = GY + 2 * n, TZ = GZ + 2 * n;
   static constexpr int TP = TX | 1;  // odd row pitch
   // plane pitch = W*TP (mod 32): row (jy, jz) starts in bank TP*(jy + W*jz)
   // mod 32, distinct for 32 consecutive (jy, jz)
-  static constexpr int ZP = ((TY * TP + 31) / 32) * 32 + ((W * TP) % 32);
+  static constexpr int ZP = TY * TP + ((W - TY) * TP % 32 + 32) % 32;
   static constexpr int NW = NT / 32;
   static constexpr int APW = 32 / GL;  // atoms per warp at a time
+  static constexpr int NROW = (W * W + GL - 1) / GL * GL;  // rows, padded to whole steps
   static constexpr size_t bytes =
-      sizeof(CT) * (TZ * ZP + NW * APW * 9 * kWPad) + sizeof(int) * NW * APW * W * W;
+      sizeof(CT) * (TZ * ZP + NW * APW * 9 * kWPad) + sizeof(int) * NROW;
 };
+
+// The (2n+1)^2 stencil rows (jy, jz) in the order in which the gather's groups of GL
+// lanes take them, the same for every atom: entries (tile offset << 8 | jz << 4 | jy),
+// first the rows that an atom may have inside its sphere, in (jz, jy) order so that a
+// step's rows start in different banks, of them the rarest last; then the rows out
+// of reach.  A row's least distance from an atom is (|j - n| - 1/2) h per axis when
+// the atom lies within half a cell of its stencil centre; 0.01 h of slack covers
+// the rounding of the centre.  Returns through n_step[0] the steps every atom takes,
+// [1] the steps that hold rows within reach.  One warp.
+template <int W, int GL>
+__device__ __forceinline__ void gather_rows(int TP, int ZP, float hy, float hz, float rcut2,
+                                            int* __restrict__ rows, int* n_step) {
+  constexpr int n = (W - 1) / 2, NP = (W * W + 31) / 32;
+  constexpr int NROW = (W * W + GL - 1) / GL * GL;
+  const int lane = threadIdx.x & 31;
+  float m[NP];  // squared least distance
+#pragma unroll
+  for (int t = 0; t < NP; t++) {
+    const int p = t * 32 + lane, jz = p / W, jy = p - jz * W;
+    const float dy = fmaxf(0.f, fabsf((float)(jy - n)) - 0.51f) * hy,
+                dz = fmaxf(0.f, fabsf((float)(jz - n)) - 0.51f) * hz;
+    m[t] = p < W * W ? dy * dy + dz * dz : 3.0e38f;
+  }
+  auto count = [&](float lim) {
+    int c = 0;
+#pragma unroll
+    for (int t = 0; t < NP; t++) c += __popc(__ballot_sync(0xffffffffu, m[t] < lim));
+    return c;
+  };
+  const int nc = count(rcut2);
+  // the farthest rows, which few atoms reach, go last: at least as many as fill the
+  // last, incomplete step, which a vote then mostly skips
+  float lim = rcut2;
+  int ncommon = nc;
+  for (int k = 1; k <= 16 && ncommon > nc / GL * GL; k++) {
+    lim = rcut2 * (1.f - 0.02f * (float)k);
+    ncommon = count(lim);
+  }
+  int at[3] = {0, ncommon, nc};
+#pragma unroll
+  for (int t = 0; t < NP; t++) {
+    const int p = t * 32 + lane, jz = p / W, jy = p - jz * W;
+    const int cls = m[t] < lim ? 0 : m[t] < rcut2 ? 1 : p < W * W ? 2 : 3;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const unsigned b = __ballot_sync(0xffffffffu, cls == c);
+      if (cls == c)
+        rows[at[c] + __popc(b & ((1u << lane) - 1u))] =
+            ((jz * ZP + jy * TP) << 8) | (jz << 4) | jy;
+      at[c] += __popc(b);
+    }
+  }
+  // table entry 15 lies outside every sphere
+  for (int i = W * W + lane; i < NROW; i += 32) rows[i] = 15;
+  if (lane == 0) {
+    n_step[0] = ncommon / GL;
+    n_step[1] = (nc + GL - 1) / GL;
+  }
+}
 
 // The gather of the atoms of one brick by a block of NT threads.  kGatherLanes
 // lanes share one atom (two atoms per warp at 16): each group builds its
-// atom's weight tables, compacts the (y, z) rows that meet the sphere and sums
-// them, one row per lane and iteration, in the order of the row list.  GL
-// lanes per atom (16 by default; the batched launch may take 8).
-template <typename CT, int W, int NT = kGatherThreads, int GL = kGatherLanes>
+// atom's weight tables and sums the rows of the block's row list, one row per lane
+// and step.  GL lanes per atom (16 by default; the batched launch may take 8).
+// A list of the rows inside each atom's own sphere (96 to 101 of 169 at n = 6) saves
+// no step over the 113 rows that any atom can reach, whose last step holds one rare
+// row, and cost nine groups of dependent loads, votes and stores per atom pair: without
+// it the mixed kernel takes 94 registers instead of 121 (80 under the bound, so that
+// 24 warps fit an SM instead of 16) and 262,143 charges on 144^3 0.199 -> 0.165 ms;
+// the FP64 one 0.395 -> 0.305 ms, of which the 12 warps instead of 8 are half.
+template <typename CT, int W, int NT = kGatherThreads, int GL = kGatherLanes, int GY = kGY,
+          int GZ = kGZ>
 __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __restrict__ sorted,
                                              const int* __restrict__ perm,
                                              const int* __restrict__ start, const BinLayout& b,
@@ -435,28 +502,29 @@ __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __re
                                              double outscale, double* __restrict__ fx,
                                              double* __restrict__ fy, double* __restrict__ fz,
                                              int bxi, int byi, int bzi, unsigned char* gsm) {
-  typedef GatherGeom<CT, W, NT, GL> GG;
+  typedef GatherGeom<CT, W, NT, GL, GY, GZ> GG;
   constexpr int n = GG::n, TX = GG::TX, TY = GG::TY, TZ = GG::TZ, TP = GG::TP, ZP = GG::ZP;
   constexpr int NW = GG::NW, APW = GG::APW;
-  constexpr int NR = kGY * kGZ;  // cell rows of the brick
-  constexpr int NG = (W * W + GL - 1) / GL;
+  constexpr int NR = GY * GZ;  // cell rows of the brick
+  static_assert(W <= 15 && kWPad == 16, "table entry 15 is free");
   static_assert(TZ * ZP < (1 << 23), "tile offsets fit the row list entries");
   typedef typename Vec4<CT>::type V;
   CT* tile = (CT*)gsm;                                   // [TZ][ZP]
   CT* tabs = tile + TZ * ZP;                             // [NW][APW][axis][d, d^2, w][kWPad]
-  int* rowl = (int*)(tabs + NW * APW * 9 * kWPad);       // [NW][APW][W*W]
+  int* rlist = (int*)(tabs + NW * APW * 9 * kWPad);      // [NROW]
+  __shared__ int n_step[2];
   __shared__ int rng_a[NR], rng_p[NR + 1];
   __shared__ int alist[kGatherList];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int grp = lane / GL, gl = lane % GL;
-  const int x0 = bxi * kGX, y0 = byi * kGY, z0 = bzi * kGZ;
-  const int ex = min(kGX, b.M[0] - x0), ey = min(kGY, b.M[1] - y0), ez = min(kGZ, b.M[2] - z0);
+  const int x0 = bxi * kGX, y0 = byi * GY, z0 = bzi * GZ;
+  const int ex = min(kGX, b.M[0] - x0), ey = min(GY, b.M[1] - y0), ez = min(GZ, b.M[2] - z0);
 
   // atoms of the brick: one range per (y, z) cell row
   int cnt = 0;
   if (tid < NR) {
-    const int yy = tid % kGY, zz = tid / kGY;
+    const int yy = tid % GY, zz = tid / GY;
     int a0 = 0, a1 = 0;
     if (yy < ey && zz < ez) {
       const int rowkey = ((z0 + zz) * b.M[1] + (y0 + yy)) * b.nbx;
@@ -475,34 +543,14 @@ __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __re
   // potential of the brick plus halo, staged by asynchronous element copies
   // so that a warp keeps all of its rows in flight
   stage_tile_async<CT, TX, TY, TZ, TP, ZP, NW>(phi, b, x0, y0, z0, n, tile);
+  if (warp == NW - 1)
+    gather_rows<W, GL>(TP, ZP, (float)s.h[1], (float)s.h[2], (float)s.rcut2, rlist, n_step);
+  CT* tb = tabs + (warp * APW + grp) * 9 * kWPad;  // [axis][d, d^2, w][j]
+  if (gl < 9) tb[gl * kWPad + 15] = gl % 3 == 1 ? (CT)3.0e38 : (CT)0;
+  if (GL < 9 && gl == 0) tb[8 * kWPad + 15] = (CT)0;
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-
-  CT* tb = tabs + (warp * APW + grp) * 9 * kWPad;  // [axis][d, d^2, w][j]
-  int* rl = rowl + (warp * APW + grp) * W * W;
-  // (jy, jz) of the rows each lane tests, the same for every atom: first the
-  // (W-1)^2 rows with jy, jz >= 1, then the 2W-1 rows with jy = 0 or jz = 0,
-  // which lie outside the sphere whenever dy^2 (dz^2) at index 0 is at least
-  // rcut^2 -- for every atom when n h exceeds rcut by more than rounding
-  constexpr int NI = (W - 1) * (W - 1);
-  constexpr int NGI = (NI + GL - 1) / GL;  // groups that hold the inner rows
-  // (jy, jz) of candidate row r (formed where it is used: a table of them
-  // would hold 2 NG registers through the whole atom loop)
-  auto cand = [&](int r, int& jy, int& jz) {
-    if (r < NI) {
-      jz = 1 + r / (W - 1);
-      jy = 1 + r % (W - 1);
-    } else if (r < NI + W) {
-      jz = r - NI;
-      jy = 0;
-    } else if (r < W * W) {
-      jz = 0;
-      jy = r - NI - W + 1;
-    } else {
-      jz = jy = 0;
-    }
-  };
-  const unsigned gmask = GL == 32 ? 0xffffffffu : ((1u << GL) - 1u);
+  const int always = n_step[0], reach = n_step[1];
   for (int c0 = 0; c0 < natoms; c0 += kGatherList) {
     brick_atom_list<NT, NR>(rng_a, rng_p, natoms, c0, kGatherList, alist);
     __syncthreads();
@@ -527,12 +575,14 @@ __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __re
       const CT pos3[3] = {a.x, a.y, a.z};
       const int org[3] = {x0, y0, z0};
       int loc[3];
+      bool far = false;  // farther than half a cell (and rounding) from its centre
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         const int c = centre_cell(pos3[d], s.inv_h[d]);
         loc[d] = wrap1(c, s.M[d]) - org[d];  // first stencil cell in tile coordinates
         for (int j = gl; j < W; j += GL) {
           const CT dd = sub_rn(pos3[d], mul_rn((CT)(c - n + j), s.h[d]));
+          if (d > 0 && j == n) far |= !(fabs(dd) <= (CT)0.505 * s.h[d]);
           const CT d2 = mul_rn(dd, dd);
           tb[(d * 3 + 0) * kWPad + j] = dd;
           tb[(d * 3 + 1) * kWPad + j] = d2;
@@ -540,28 +590,8 @@ __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __re
         }
       }
       __syncwarp();
-      // the rows with jy = 0 or jz = 0 are tested only when one of the warp's
-      // atoms could have one inside (adding dz^2 >= 0 cannot take a sum below
-      // dy^2, so dy^2 >= rcut^2 at jy = 0 rules out its whole plane)
-      const bool edges = !__all_sync(0xffffffffu, tb[(1 * 3 + 1) * kWPad + 0] >= s.rcut2 &&
-                                                      tb[(2 * 3 + 1) * kWPad + 0] >= s.rcut2);
-      // non-empty rows (the whole row is outside the sphere when dy^2+dz^2 >= rcut^2)
-      int nrow = 0;
-#pragma unroll
-      for (int g = 0; g < NG; g++) {
-        if (g >= NGI && !edges) break;  // warp-uniform
-        const int r = g * GL + gl;
-        int jy, jz;
-        cand(r, jy, jz);
-        bool ne = false;
-        if (r < W * W)
-          ne = add_rn(tb[(1 * 3 + 1) * kWPad + jy], tb[(2 * 3 + 1) * kWPad + jz]) < s.rcut2;
-        const unsigned m = (__ballot_sync(0xffffffffu, ne) >> (GL * grp)) & gmask;
-        // the row's tile offset with its (jz, jy): bits 8+ offset, 4-7 jz, 0-3 jy
-        if (ne) rl[nrow + __popc(m & ((1u << gl) - 1u))] = ((jz * ZP + jy * TP) << 8) | (jz << 4) | jy;
-        nrow += __popc(m);
-      }
-      __syncwarp();
+      // coordinates so large that their rounding moves the centre: all rows
+      const int steps = __any_sync(0xffffffffu, far) ? GG::NROW / GL : reach;
       CT dx2[W], wx[W], wdx[W];
 #pragma unroll
       for (int k = 0; k < W; k++) {
@@ -569,7 +599,7 @@ __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __re
         wx[k] = tb[(0 * 3 + 2) * kWPad + k];
         wdx[k] = wx[k] * tb[(0 * 3 + 0) * kWPad + k];
       }
-      // each row's 2n+1 terms and a lane's rows (about rows/16 of them) in CT, the
+      // each row's 2n+1 terms and a lane's rows (seven at n = 6) in CT, the
       // lanes' sums in double (the reference's AT)
       CT lx = 0, ly = 0, lz = 0;
       const CT* abase = tile + loc[2] * ZP + loc[1] * TP + loc[0];  // the atom's first row
@@ -582,11 +612,13 @@ __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __re
       auto rows = [&](auto k0, auto k1) {
         constexpr int K0 = decltype(k0)::value;
         constexpr int K1 = decltype(k1)::value;
-        for (int i = gl; i < nrow; i += GL) {
-          const int r = rl[i];
+        for (int i = 0; i < steps; i++) {
+          const int r = rlist[i * GL + gl];
           const int jz = (r >> 4) & 15, jy = r & 15;
           const CT dy2 = tb[(1 * 3 + 1) * kWPad + jy], dz2 = tb[(2 * 3 + 1) * kWPad + jz];
           const CT rem = s.rcut2 - (dy2 + dz2);
+          // adding dx^2 >= 0 cannot take the sum below dy^2 + dz^2
+          if (i >= always && !__any_sync(0xffffffffu, add_rn(dy2, dz2) < s.rcut2)) continue;
           const CT* row = abase + (r >> 8);
           CT s0, s1;
           row_sums<CT, W, K0, K1>(row, dx2, wx, wdx, dy2, dz2, rem, s.rcut2, s0, s1);
@@ -621,7 +653,7 @@ __device__ __forceinline__ void gather_brick(const typename Vec4<CT>::type* __re
   }
 }
 
-template <typename CT, int W>
+template <typename CT, int W, int GY, int GZ>
 __global__ void __launch_bounds__(kGatherThreads, sizeof(CT) == 4 ? 2 : 1)
     k_gather_tiled(const typename Vec4<CT>::type* __restrict__ sorted,
                    const int* __restrict__ perm, const int* __restrict__ start, BinLayout b,
@@ -629,8 +661,9 @@ __global__ void __launch_bounds__(kGatherThreads, sizeof(CT) == 4 ? 2 : 1)
                    double* __restrict__ fx, double* __restrict__ fy, double* __restrict__ fz) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char gsm[];
-  gather_brick<CT, W>(sorted, perm, start, b, s, phi, outscale, fx, fy, fz, blockIdx.x,
-                      blockIdx.y, blockIdx.z, gsm);
+  gather_brick<CT, W, kGatherThreads, kGatherLanes, GY, GZ>(sorted, perm, start, b, s, phi,
+                                                            outscale, fx, fy, fz, blockIdx.x,
+                                                            blockIdx.y, blockIdx.z, gsm);
 }
 
 // ===========================================================================
@@ -714,28 +747,51 @@ bool spread_tiled_supported(const Stencil<CT>& s) {
   return W == 9 || W == 11 || W == 13 || W == 15;
 }
 
-template <typename CT, int W>
-static cudaError_t gather_w(const typename Vec4<CT>::type* sorted, const int* perm,
-                            const int* start, const BinLayout& b, const Stencil<CT>& s,
-                            const CT* phi, double outscale, double* fx, double* fy, double* fz,
-                            bool pdl, cudaStream_t st) {
-  const size_t smem = GatherGeom<CT, W>::bytes;
+template <typename CT, int W, int GY, int GZ>
+static cudaError_t gather_shape(const typename Vec4<CT>::type* sorted, const int* perm,
+                                const int* start, const BinLayout& b, const Stencil<CT>& s,
+                                const CT* phi, double outscale, double* fx, double* fy,
+                                double* fz, bool pdl, cudaStream_t st) {
+  const size_t smem = GatherGeom<CT, W, kGatherThreads, kGatherLanes, GY, GZ>::bytes;
   static std::atomic<bool> attr[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (!attr[dev]) {
     const cudaError_t e = cudaFuncSetAttribute(
-        k_gather_tiled<CT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_gather_tiled<CT, W, GY, GZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     attr[dev] = true;
   }
-  dim3 grd((b.M[0] + kGX - 1) / kGX, (b.M[1] + kGY - 1) / kGY, (b.M[2] + kGZ - 1) / kGZ);
-  const cudaError_t e = launch_dependent(pdl, k_gather_tiled<CT, W>, grd, dim3(kGatherThreads),
-                                         smem, st, sorted, perm, start, b, s, phi, outscale, fx,
-                                         fy, fz);
+  dim3 grd((b.M[0] + kGX - 1) / kGX, (b.M[1] + GY - 1) / GY, (b.M[2] + GZ - 1) / GZ);
+  const cudaError_t e = launch_dependent(pdl, k_gather_tiled<CT, W, GY, GZ>, grd,
+                                         dim3(kGatherThreads), smem, st, sorted, perm, start, b,
+                                         s, phi, outscale, fx, fy, fz);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
+}
+
+template <typename CT, int W>
+static cudaError_t gather_w(const typename Vec4<CT>::type* sorted, const int* perm,
+                            const int* start, const BinLayout& b, const Stencil<CT>& s,
+                            const CT* phi, double outscale, double* fx, double* fy, double* fz,
+                            bool pdl, cudaStream_t st) {
+  // the smallest brick whose blocks all run at about once (two per SM in the mixed form,
+  // one in FP64): a grid of few bricks is bound by one brick's time.  Gather stage in
+  // us with 16 x 16 x 8, 16 x 8 x 8 and 16 x 8 x 4 cells: mixed 38^3 (45, 75, 150
+  // bricks) 33, 23, 18; 64^3 (128, 256, 512) 35, 31, 32; 80^3 (250, 500, 1000) 47, 49,
+  // 56; 144^3 169, 185, -; FP64 38^3 43, 29, 21; 64^3 45, 48, 54
+  const int slots = (sizeof(CT) == 4 ? 2 : 1) * sm_count() * 9 / 8;
+  auto bricks = [&](int gy, int gz) {
+    return (long long)((b.M[0] + kGX - 1) / kGX) * ((b.M[1] + gy - 1) / gy) *
+           ((b.M[2] + gz - 1) / gz);
+  };
+  if (bricks(8, 4) <= slots)
+    return gather_shape<CT, W, 8, 4>(sorted, perm, start, b, s, phi, outscale, fx, fy, fz, pdl, st);
+  if (bricks(8, 8) <= slots)
+    return gather_shape<CT, W, 8, 8>(sorted, perm, start, b, s, phi, outscale, fx, fy, fz, pdl, st);
+  return gather_shape<CT, W, kGY, kGZ>(sorted, perm, start, b, s, phi, outscale, fx, fy, fz, pdl,
+                                       st);
 }
 
 template <typename CT>

@@ -15,7 +15,7 @@ namespace gse {
 constexpr int kBinX64 = 4, kBinX32 = 16;
 constexpr int kWPad = 16;           // padded stencil width (2n+1 <= 15 on the tiled path)
 constexpr int kGX = 16, kGY = 16, kGZ = 8;  // gather brick (cells); kGX multiple of kBinX32
-constexpr int kGatherThreads = 256;          // >= kGY * kGZ
+constexpr int kGatherThreads = 384;          // >= kGY * kGZ
 constexpr int kGatherLanes = 16;             // lanes sharing one atom in the gather
 constexpr int kMinTiledGrid = 10;   // smallest grid side on the tiled path
 constexpr int kSB = 16;             // scatter-spread brick (cells per axis)
