@@ -223,7 +223,8 @@ template <int W, int NT>
 __device__ __forceinline__ void adj_scatter_brick(
     const float4* __restrict__ sorted, const float4* __restrict__ gs,
     const int* __restrict__ start, const BinLayout& b, const Stencil<float>& s, float cA, int bxi,
-    int byi, int bzi, int* __restrict__ tile, long long* __restrict__ grid64) {
+    int byi, int bzi, int* __restrict__ tile, long long* __restrict__ grid64, int part = 0,
+    int nparts = 1) {
   typedef ScatterGeom<W> G;
   constexpr int n = G::n;
   constexpr int NW = NT / 32;
@@ -254,7 +255,7 @@ __device__ __forceinline__ void adj_scatter_brick(
     brick_atom_list<NT, kSB * kSB>(rng_a, rng_p, total, c0, kScatterList, alist);
     __syncthreads();
     const int nc = min(kScatterList, total - c0);
-    for (int q = warp; q < nc; q += NW) {
+    for (int q = warp + part * NW; q < nc; q += NW * nparts) {
       const int ai = alist[q];
       const float4 a = sorted[ai];
       const float4 gv = gs[ai];
@@ -620,10 +621,11 @@ template <int W>
 __global__ void __launch_bounds__(kAdjScatterThreads, 2)
     k_adj_scatter(const float4* __restrict__ sorted, const float4* __restrict__ gs,
                   const int* __restrict__ start, BinLayout b, Stencil<float> s, float cA,
-                  long long* __restrict__ grid64) {
+                  int nparts, long long* __restrict__ grid64) {
   extern __shared__ int atile[];
-  adj_scatter_brick<W, kAdjScatterThreads>(sorted, gs, start, b, s, cA, blockIdx.x, blockIdx.y,
-                                           blockIdx.z, atile, grid64);
+  adj_scatter_brick<W, kAdjScatterThreads>(sorted, gs, start, b, s, cA, blockIdx.x / nparts,
+                                           blockIdx.y, blockIdx.z, atile, grid64,
+                                           blockIdx.x % nparts, nparts);
 }
 
 template <int W>
@@ -703,9 +705,11 @@ cudaError_t adj_scatter_w(const float4* sorted, const float4* gs, const int* sta
   const long long size = (long long)b.M[0] * b.M[1] * b.M[2];
   e = cudaMemsetAsync(grid64, 0, sizeof(long long) * size, st);
   if (e != cudaSuccess) return e;
-  const dim3 grd((b.M[0] + kSB - 1) / kSB, (b.M[1] + kSB - 1) / kSB, (b.M[2] + kSB - 1) / kSB);
-  k_adj_scatter<W><<<grd, kAdjScatterThreads, smem, st>>>(sorted, gs, start, b, s,
-                                                          (float)(c * (double)s.pref), grid64);
+  dim3 grd((b.M[0] + kSB - 1) / kSB, (b.M[1] + kSB - 1) / kSB, (b.M[2] + kSB - 1) / kSB);
+  const int nparts = scatter_parts((long long)grd.x * grd.y * grd.z);
+  grd.x *= nparts;
+  k_adj_scatter<W><<<grd, kAdjScatterThreads, smem, st>>>(
+      sorted, gs, start, b, s, (float)(c * (double)s.pref), nparts, grid64);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_grid64_to_real(grid64, size, lambda, st);

@@ -242,7 +242,8 @@ __device__ __forceinline__ void scatter_brick(const float4* __restrict__ sorted,
                                               const int* __restrict__ start, const BinLayout& b,
                                               const Stencil<float>& s, int bxi, int byi, int bzi,
                                               int* __restrict__ tile,
-                                              long long* __restrict__ grid64) {
+                                              long long* __restrict__ grid64, int part = 0,
+                                              int nparts = 1) {
   typedef ScatterGeom<W> G;
   constexpr int n = G::n;
   constexpr int NT = kScatterThreads, NW = NT / 32;
@@ -275,7 +276,7 @@ __device__ __forceinline__ void scatter_brick(const float4* __restrict__ sorted,
     brick_atom_list<NT, kSB * kSB>(rng_a, rng_p, total, c0, kScatterList, alist);
     __syncthreads();
     const int nc = min(kScatterList, total - c0);
-    for (int q = warp; q < nc; q += NW) {
+    for (int q = warp + part * NW; q < nc; q += NW * nparts) {
       const float4 a = sorted[alist[q]];
       const float pos3[3] = {a.x, a.y, a.z};
       const int org[3] = {x0, y0, z0};
@@ -351,11 +352,13 @@ __device__ __forceinline__ void scatter_brick(const float4* __restrict__ sorted,
 template <int W>
 __global__ void __launch_bounds__(kScatterThreads)
     k_spread_scatter(const float4* __restrict__ sorted, const int* __restrict__ start,
-                     BinLayout b, Stencil<float> s, long long* __restrict__ grid64) {
+                     BinLayout b, Stencil<float> s, int nparts,
+                     long long* __restrict__ grid64) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ int tile[];
-  scatter_brick<W>(sorted, start, b, s, blockIdx.x, blockIdx.y, blockIdx.z, tile, grid64);
+  scatter_brick<W>(sorted, start, b, s, blockIdx.x / nparts, blockIdx.y, blockIdx.z, tile, grid64,
+                   blockIdx.x % nparts, nparts);
 }
 
 // float grid from the int64 accumulation grid at 2^kFlushBits
@@ -840,8 +843,9 @@ static cudaError_t scatter_w(const float4* sorted, const int* start, const BinLa
   const int nb[3] = {(b.M[0] + kSB - 1) / kSB, (b.M[1] + kSB - 1) / kSB,
                      (b.M[2] + kSB - 1) / kSB};
   // with the grid cleared earlier the spread follows the binning's last kernel
-  e = launch_dependent(zeroed, k_spread_scatter<W>, dim3(nb[0], nb[1], nb[2]),
-                       dim3(kScatterThreads), smem, st, sorted, start, b, s, grid64);
+  const int nparts = scatter_parts((long long)nb[0] * nb[1] * nb[2]);
+  e = launch_dependent(zeroed, k_spread_scatter<W>, dim3(nb[0] * nparts, nb[1], nb[2]),
+                       dim3(kScatterThreads), smem, st, sorted, start, b, s, nparts, grid64);
   if (e != cudaSuccess) return e;
   // rho == nullptr: the caller converts the int64 grid itself (the own FFT)
   if (rho) k_grid64_to_real<<<sm_count() * 8, 256, 0, st>>>(grid64, size, rho);

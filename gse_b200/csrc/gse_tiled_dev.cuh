@@ -64,6 +64,18 @@ struct ScatterGeom {
 
 constexpr int kMinShift = 11;   // 2^30 * 2^(40-11) * 8 overlapping tiles < 2^63
 
+// Blocks per brick of a scatter launch of `bricks` bricks (at two blocks per SM): each
+// takes every nparts-th round of the brick's atoms in a tile of its own at the whole
+// brick's scale, so that the grid is the same bit for bit.  As many as fill the SMs
+// once: a second wave of blocks repeats the tile's clearing and flush.  Spread stage
+// in us with 1, 2, 4, 8 blocks per brick: 24^3 (8 bricks) 54, 44, 33, 29; 38^3 (27) 53,
+// 40, 32, 30; 64^3 (64) 51, 39, 35, 43; 80^3 (125) 52, 49, 57, 70; 144^3 (729) 154,
+// 174, 224, -.
+inline int scatter_parts(long long bricks) {
+  const long long most = 2LL * sm_count() / (bricks > 0 ? bricks : 1);
+  return (int)(most < 1 ? 1 : most > 8 ? 8 : most);
+}
+
 // Block prologue of a scatter brick: the brick's atoms (one contiguous range
 // per (y, z) cell row, start offsets in rng_a, exclusive prefix in rng_p),
 // the cleared tile, and the brick's power-of-two scale 2^S such that the sum
@@ -103,10 +115,15 @@ __device__ __forceinline__ int brick_prologue(const int* __restrict__ start, con
   // magnitudes, so the scale does not depend on the order of a bin's atoms
   double qs = 0.0;
   float qm = 0.f;
-  for (int j = 0; j < cnt; j++) {
-    const float q = bound(a0 + j);
-    qs += (double)q;
-    qm = fmaxf(qm, q);
+  for (int j = 0; j < cnt; j += 4) {  // four loads in flight
+    float q[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) q[k] = j + k < cnt ? bound(a0 + j + k) : 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      qs += (double)q[k];
+      qm = fmaxf(qm, q[k]);
+    }
   }
   qs = warp_sum(qs);
 #pragma unroll
@@ -125,16 +142,16 @@ __device__ __forceinline__ int brick_prologue(const int* __restrict__ start, con
     }
     const double sum_b = q * 1.0001 + 1e-30;
     const double one_b = (double)m * 1.0001 + 1e-30;
-    int sh = kFlushBits;
-    while (sh > kMinShift && (sum_b * exp2((double)sh) >= 1073741824.0 ||
-                              one_b * exp2((double)sh) >= 4194304.0))
-      sh--;
+    // the largest sh <= kFlushBits with sum_b 2^sh < 2^30 and one_b 2^sh < 2^22, by the
+    // exponents (a NaN sum, which the binning reports, bounds nothing)
+    auto exponent = [](double v) { return ((__double2hiint(v) >> 20) & 0x7ff) - 1023; };
+    int sh = min(kFlushBits, 21 - exponent(one_b));
+    if (!isnan(sum_b)) sh = min(sh, 29 - exponent(sum_b));
     // even the coarsest scale leaves the tile's int32 sums without headroom:
     // the brick's result would wrap, so the call reports a range error
     // (non-finite charges are the binning's report)
-    if ((sum_b * exp2((double)sh) >= 1073741824.0 || one_b * exp2((double)sh) >= 4194304.0) &&
-        isfinite(sum_b) && b.flags)
-      *b.flags = kFlagRange;
+    if (sh < kMinShift && isfinite(sum_b) && b.flags) *b.flags = kFlagRange;
+    sh = max(sh, kMinShift);
     s_shift = sh;
   }
   __syncthreads();
