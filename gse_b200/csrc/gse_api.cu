@@ -216,6 +216,12 @@ struct gse_context {
   cudaGraphExec_t fwd_exec = nullptr;
   long long fwd_launches = 0;
   bool fwd_graphs = true;
+  // calls of one key that run directly before the next is captured: one, and more
+  // after graphs that were dropped again before they had repaid their capture
+  int fwd_seen = 0, fwd_need = 1, fwd_replays = 0;
+  // the legacy default stream cannot be captured: calls on it are captured on this
+  // stream and the graph is launched into theirs
+  cudaStream_t cap_stream = nullptr;
   // classification of the pointers of the captured call, for the replay path
   bool fwd_host_io = false, fwd_e_host = false;
   const double* fwd_e_raw = nullptr;
@@ -297,6 +303,16 @@ gse_status_t check_stencil(const gse_context_t* c, const double box[3], double s
       return fail(GSE_ERR_STENCIL_TOO_LARGE, "stencil 2n+1=%d exceeds %d on axis %d", 2 * n + 1,
                   kMaxStencil, d);
   }
+  return GSE_OK;
+}
+
+// All work of the context on `st` from here on.
+gse_status_t use_stream(gse_context_t* c, cudaStream_t st) {
+  if (c->stream == st) return GSE_OK;
+  c->stream = st;
+  CUFFT(cufftSetStream(c->plan_f, st));
+  CUFFT(cufftSetStream(c->plan_b, st));
+  if (c->green_cb) CUFFT(cufftSetStream(c->plan_bg, st));
   return GSE_OK;
 }
 
@@ -949,6 +965,7 @@ gse_status_t gse_destroy(gse_context_t* c) {
     cufftDestroy(c->plan_b);
   }
   if (c->green_cb) cufftDestroy(c->plan_bg);
+  if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
   cudaFree(c->d_rho);
   cudaFree(c->d_phi);
   cudaFree(c->d_rhok);
@@ -982,12 +999,9 @@ gse_status_t gse_destroy(gse_context_t* c) {
 
 gse_status_t gse_set_stream(gse_context_t* c, void* stream) {
   TRY(check_ctx(c));
+  if (c->stream == (cudaStream_t)stream) return GSE_OK;
   drop_fwd_graph(c);
-  c->stream = (cudaStream_t)stream;
-  CUFFT(cufftSetStream(c->plan_f, c->stream));
-  CUFFT(cufftSetStream(c->plan_b, c->stream));
-  if (c->green_cb) CUFFT(cufftSetStream(c->plan_bg, c->stream));
-  return GSE_OK;
+  return use_stream(c, (cudaStream_t)stream);
 }
 
 gse_status_t gse_set_box(gse_context_t* c, double bx, double by, double bz) {
@@ -1151,6 +1165,7 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
     }
     if ((he ? reinterpret_cast<double*>(uintptr_t(1)) : energy) == k.e) {
       CU(cudaGraphLaunch(c->fwd_exec, c->stream));
+      c->fwd_replays++;
       c->launches += c->fwd_launches;
       c->rho_valid = c->phi_valid = c->energy_valid = true;
       c->fwd_e_raw = energy;
@@ -1165,8 +1180,8 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
   TRY(check_xyz(c->p.device, fx, fy, fz, "force array"));
   // Graph replay applies to calls whose positions and forces are device or
   // page-locked host memory (the copies to and from the host then sit in the
-  // graph), on a stream that can be captured, without stage timing; the key
-  // (pointers, count, box, stream) must repeat exactly.  A host energy is read
+  // graph), without stage timing; the key (pointers, count, box, stream) must
+  // repeat exactly.  A host energy is read
   // through the context's page-locked scalar after the call has finished.
   auto io_ok = [](const void* p) { return is_device_ptr(p) || is_pinned_host(p); };
   const bool host_e = energy && !is_device_ptr(energy);
@@ -1174,8 +1189,8 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
                                                  io_ok(fz));
   const bool host_io = host_e || (fx && !is_device_ptr(fx)) || (fy && !is_device_ptr(fy)) ||
                        (fz && !is_device_ptr(fz));
-  const bool graphable = c->fwd_graphs && !c->timing && c->stream != nullptr && n > 0 &&
-                         io_ok(xyzq) && forces_ok && c->gtab_valid;
+  const bool graphable = c->fwd_graphs && !c->timing && n > 0 && io_ok(xyzq) && forces_ok &&
+                         c->gtab_valid;
   gse_context_t::FwdKey key;
   key.n = n;
   key.x = xyzq;
@@ -1212,23 +1227,46 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
   };
   if (c->fwd_exec && key == c->fwd_key) {
     CU(cudaGraphLaunch(c->fwd_exec, c->stream));
+    c->fwd_replays++;
     c->launches += c->fwd_launches;
     c->rho_valid = c->phi_valid = c->energy_valid = true;
     return done(host_io);
   }
   if (!(key == c->fwd_key)) {
-    // first call with this key: run it directly and remember the key
+    // first call with this key: run it directly and remember the key.  A capture costs
+    // some ten calls; a program whose buffers change sooner than that is left alone
+    // for longer each time.
+    if (c->fwd_exec) c->fwd_need = c->fwd_replays >= 16 ? 1 : std::min(64, 4 * c->fwd_need);
     drop_fwd_graph(c);
     TRY(body(&host));
     c->fwd_key = key;
+    c->fwd_seen = 1;
     return done(host);
   }
-  // second identical call: capture, instantiate, launch
+  if (c->fwd_seen < c->fwd_need) {
+    c->fwd_seen++;
+    TRY(body(&host));
+    return done(host);
+  }
+  // the next identical call: capture, instantiate, launch
   const long long l0 = c->launches;
-  CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  const gse_status_t st = body(&host);
+  const cudaStream_t user = c->stream;
+  if (!user) {
+    if (!c->cap_stream)
+      CU(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
+    TRY(use_stream(c, c->cap_stream));
+  }
   cudaGraph_t g = nullptr;
-  const cudaError_t ec = cudaStreamEndCapture(c->stream, &g);
+  gse_status_t st = GSE_OK;
+  cudaError_t ec = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+  if (ec == cudaSuccess) {
+    st = body(&host);
+    ec = cudaStreamEndCapture(c->stream, &g);
+  } else if (user) {
+    return fail(GSE_ERR_CUDA, "cudaStreamBeginCapture: %s", cudaGetErrorString(ec));
+  }
+  TRY(use_stream(c, user));
+  c->fwd_replays = 0;
   gse_status_t result = st;
   if (st == GSE_OK && ec == cudaSuccess) {
     const cudaError_t ei = cudaGraphInstantiate(&c->fwd_exec, g, 0);
