@@ -255,13 +255,15 @@ gse_status_t gse_adjoint(gse_context_t* ctx, int n, const void* xyzq, double dLd
                          double* dx, double* dy, double* dz);
 
 /* ---- Ewald reference sum --------------------------------------------------- */
+/* The two calls below take their scratch from a memory pool of the library's own,
+ * one per device, which keeps up to 256 MB between calls.  They synchronise the
+ * stream; calls of several threads and streams may overlap. */
 
 /* CpuEwaldRecip::calcForceEnergy (CpuEwaldRecip.cpp:87-147) on the GPU in FP64:
  * E = sum over integer k != 0 with |k|^2 <= kcut^2 of
  * (2 pi / V) ccelec exp(-sigma^2 |k|^2 / 2) / |k|^2 |S(k)|^2 and the forces
- * -dE/dr (force arrays may all be NULL).  Independent of any context; it
- * allocates its own scratch and returns after the results are written.
- * kcut must lie in [1, 255]. */
+ * -dE/dr (force arrays may all be NULL).  Independent of any context; returns
+ * after the results are written.  kcut must lie in [1, 255]. */
 gse_status_t gse_ewald_recip(int device, void* stream, double sigma, int kcut, double box_x,
                              double box_y, double box_z, double ccelec, int n, const double* xyzq,
                              double* energy, double* fx, double* fy, double* fz);
@@ -279,9 +281,8 @@ gse_status_t gse_ewald_recip(int device, void* stream, double sigma, int kcut, d
  * from 0) and |inb14[k]| the 1-based partner; the pair (a, b), a < b, is
  * skipped when b is listed under a.  Exclusion arrays and energy are host
  * memory; xyzq (double4 per atom) and the force arrays host or device memory.
- * Independent of any context; it allocates its own scratch and returns after
- * the results are written.  The result does not depend on the order in which
- * the GPU runs its blocks. */
+ * Independent of any context; returns after the results are written.  The
+ * result does not depend on the order in which the GPU runs its blocks. */
 gse_status_t gse_ewald_direct(int device, void* stream, double sigma, double rcut, double box_x,
                               double box_y, double box_z, double ccelec, int n, const double* xyzq,
                               int n_iblo14, const int* iblo14, const int* inb14, double* energy,
