@@ -28,132 +28,233 @@
 
 namespace gse {
 
-// lambda(r) += c q_i A e (G_i . u) over the sphere of atom i (global atomics);
-// one warp per atom.
+// ---------------------------------------------------------------------------
+// Atom-parallel kernels: the FP64 form, and the mixed form's shapes that the tiled
+// kernels do not take.  A warp per atom, its two halves on every other z plane of the
+// stencil, a lane on one x offset: the x factors stay in the lane's registers, the y
+// and z factors come from tables of the warp, both grids are read along x, and what
+// only depends on z is applied once per plane (five FP64 operations a point in the
+// source, nine in the gather).  Every lane on a point of its own, with an exponential
+// and four divisions each, took 0.31 ms for the source and 0.45 ms for the gather at
+// 23,559 charges in FP64; now 0.071 and 0.162 ms, bound by the source's reductions at L2 and
+// by the FP64 pipe and load latency at 16 warps per SM.
+// ---------------------------------------------------------------------------
+constexpr int kAdjWarps = 8;  // warps per block
+constexpr int kAdjRows = 7;   // rows of a plane whose loads are in flight together
+
 template <typename CT>
-__device__ __forceinline__ void adj_source_atom(const typename Vec4<CT>::type& a, int i,
-                                                const Stencil<CT>& s, double c,
-                                                const double* __restrict__ gfx,
-                                                const double* __restrict__ gfy,
-                                                const double* __restrict__ gfz,
-                                                CT* __restrict__ lambda) {
+struct AdjRowTab {
+  // y, z: u = x - r, u^2, e = exp(-u^2 / (2 s^2)), e u
+  CT u[2][kMaxStencil], u2[2][kMaxStencil], e[2][kMaxStencil], eu[2][kMaxStencil];
+  int off[2][kMaxStencil];  // wrapped index, along z times My
+};
+
+// Tables of one atom's y and z axes by its warp; returns its first x cell.
+template <typename CT>
+__device__ __forceinline__ int adj_tables(const CT (&pos)[3], const Stencil<CT>& s,
+                                          AdjRowTab<CT>& t) {
   const int lane = threadIdx.x & 31;
+  __syncwarp();  // the previous atom's tables are read
+#pragma unroll
+  for (int d = 1; d < 3; d++) {
+    const int c0 = round_to_int(mul_rn(pos[d], s.inv_h[d])) - s.nst[d];
+    for (int j = lane; j < 2 * s.nst[d] + 1; j += 32) {
+      const CT u = sub_rn(pos[d], mul_rn((CT)(c0 + j), s.h[d])), u2 = mul_rn(u, u);
+      const CT e = gexp(-u2 * s.inv_2s2);
+      t.u[d - 1][j] = u;
+      t.u2[d - 1][j] = u2;
+      t.e[d - 1][j] = e;
+      t.eu[d - 1][j] = e * u;
+      t.off[d - 1][j] = pmod(c0 + j, s.M[d]) * (d == 1 ? 1 : s.M[1]);
+    }
+  }
+  __syncwarp();
+  return round_to_int(mul_rn(pos[0], s.inv_h[0])) - s.nst[0];
+}
+
+// The points of the cube by planes: for each run of 16 x offsets and each plane of
+// this half-warp, plane(jz, e_x, u_x, u_x^2), then for its rows, up to kAdjRows at a
+// time, load(k, grid index) of all of them and use(k, jy), then done(jz).
+template <typename CT, class Plane, class Load, class Use, class Done>
+__device__ __forceinline__ void adj_planes(const CT (&pos)[3], const Stencil<CT>& s,
+                                           const AdjRowTab<CT>& t, int c0x, Plane plane,
+                                           Load load, Use use, Done done) {
+  const int lane = threadIdx.x & 31, xl = lane & 15, half = lane >> 4;
   const int W0 = 2 * s.nst[0] + 1, W1 = 2 * s.nst[1] + 1, W2 = 2 * s.nst[2] + 1;
-  {
-    const CT pos[3] = {a.x, a.y, a.z};
-    const CT G[3] = {(CT)gfx[i], (CT)gfy[i], (CT)gfz[i]};
-    const CT amp = (CT)(c * (double)a.w * (double)s.pref);
-    int c0[3];
+  for (int xb = xl; xb < W0; xb += 16) {
+    const CT u = sub_rn(pos[0], mul_rn((CT)(c0x + xb), s.h[0]));
+    const CT u2 = mul_rn(u, u), e = gexp(-u2 * s.inv_2s2);
+    const int x = pmod(c0x + xb, s.M[0]);
+    for (int jz = half; jz < W2; jz += 2) {
+      plane(jz, e, u, u2);
+      const long long base = x + (long long)t.off[1][jz] * s.M[0];
+      for (int j0 = 0; j0 < W1; j0 += kAdjRows) {
 #pragma unroll
-    for (int d = 0; d < 3; d++) c0[d] = round_to_int(mul_rn(pos[d], s.inv_h[d])) - s.nst[d];
-    for (int t = lane; t < W0 * W1 * W2; t += 32) {
-      const int tz = t / (W0 * W1), r = t - tz * W0 * W1, ty = r / W0, tx = r - ty * W0;
-      const int p[3] = {c0[0] + tx, c0[1] + ty, c0[2] + tz};
-      CT u[3];
+        for (int k = 0; k < kAdjRows; k++)
+          if (j0 + k < W1) load(k, base + (long long)t.off[0][j0 + k] * s.M[0]);
 #pragma unroll
-      for (int d = 0; d < 3; d++) u[d] = sub_rn(pos[d], mul_rn((CT)p[d], s.h[d]));
-      const CT r2 = add_rn(add_rn(mul_rn(u[0], u[0]), mul_rn(u[1], u[1])), mul_rn(u[2], u[2]));
-      if (r2 < s.rcut2) {
-        const CT e = gexp(-r2 * s.inv_2s2);
-        const CT v = amp * e * (G[0] * u[0] + G[1] * u[1] + G[2] * u[2]);
-        const long long idx = pmod(p[0], s.M[0]) +
-                              ((long long)pmod(p[1], s.M[1]) + (long long)pmod(p[2], s.M[2]) * s.M[1]) * s.M[0];
-        atomicAdd(lambda + idx, v);
+        for (int k = 0; k < kAdjRows; k++)
+          if (j0 + k < W1) use(k, j0 + k);
       }
+      done(jz);
     }
   }
 }
 
+// lambda(r) += c q_i A e (G_i . u) over the sphere of atom i (global atomics).
 template <typename CT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * kAdjWarps)
     k_adj_source(const typename Vec4<CT>::type* __restrict__ xyzq, const int* __restrict__ perm,
                  int n, Stencil<CT> s, double c, const double* __restrict__ gfx,
                  const double* __restrict__ gfy, const double* __restrict__ gfz,
                  CT* __restrict__ lambda) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int ii = gw; ii < n; ii += nw)
-    adj_source_atom<CT>(xyzq[ii], perm[ii], s, c, gfx, gfy, gfz, lambda);
+  __shared__ AdjRowTab<CT> tabs[kAdjWarps];
+  const int w = threadIdx.x >> 5;
+  AdjRowTab<CT>& t = tabs[w];
+  for (int ii = blockIdx.x * kAdjWarps + w; ii < n; ii += gridDim.x * kAdjWarps) {
+    const auto a = xyzq[ii];
+    const int i = perm[ii];
+    const CT pos[3] = {a.x, a.y, a.z};
+    const CT G[3] = {(CT)gfx[i], (CT)gfy[i], (CT)gfz[i]};
+    const CT amp = (CT)(c * (double)a.w * (double)s.pref);
+    const int c0x = adj_tables<CT>(pos, s, t);
+    CT t1 = 0, t2 = 0, ux2 = 0, uz2 = 0;  // of the plane
+    long long at[kAdjRows];
+    adj_planes<CT>(
+        pos, s, t, c0x,
+        [&](int jz, CT e, CT u, CT u2) {
+          const CT f = amp * e * t.e[1][jz];
+          t1 = f * (G[0] * u + G[2] * t.u[1][jz]);
+          t2 = f * G[1];
+          ux2 = u2;
+          uz2 = t.u2[1][jz];
+        },
+        [&](int k, long long idx) { at[k] = idx; },
+        [&](int k, int jy) {
+          if (add_rn(add_rn(ux2, t.u2[0][jy]), uz2) < s.rcut2)
+            atomicAdd(lambda + at[k], t1 * t.e[0][jy] + t2 * t.eu[0][jy]);
+        },
+        [](int) {});
+  }
+}
+
+// The lanes' sums of 16 values in FP64: at each step a lane keeps half of its values and
+// hands the other half to its partner (the butterfly's sums, at a quarter of its
+// shuffles).  v[0] of lanes 2 i and 2 i + 1 is the sum of value i.
+__device__ __forceinline__ void warp_sum16(double (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 8; h > 0; h >>= 1) {
+    const bool up = lane & (2 * h);
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const double give = up ? v[i] : v[i + h];
+      v[i] = (up ? v[i + h] : v[i]) + __shfl_xor_sync(0xffffffffu, give, 2 * h);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// One atom's outputs from its sums m = {P, V (3), T0, T1 (3), Mxx, Mxy, Mxz, Myy, Myz,
+// Mzz} (the cube's over Psi without the spread's prefactor, the sphere's over phi), by
+// lanes 0 to 3, which hold G: dL/dq and the three dL/dx.
+__device__ __forceinline__ void adj_outputs(const double* m, const double (&G)[3], double q,
+                                            double pref_sp, double inv_s2, double cA, int o,
+                                            double* __restrict__ dq, double* __restrict__ dx,
+                                            double* __restrict__ dy, double* __restrict__ dz) {
+  const int lane = threadIdx.x & 31;
+  // lane 0: T1 . G; lane 1 + d: row d of M times G
+  const int i0 = lane == 0 ? 5 : 7 + lane, i1 = lane == 0 ? 6 : lane == 1 ? 9 : 9 + lane,
+            i2 = lane == 0 ? 7 : lane == 1 ? 10 : 10 + lane;
+  const double t = m[i0] * G[0] + m[i1] * G[1] + m[i2] * G[2];
+  const double Gd = lane == 1 ? G[0] : lane == 2 ? G[1] : G[2];
+  double* out = lane == 0 ? dq : lane == 1 ? dx : lane == 2 ? dy : dz;
+  // (r - x) = -u
+  out[o] = lane == 0 ? pref_sp * m[0] + cA * t
+                     : -q * pref_sp * inv_s2 * m[lane] + cA * q * (Gd * m[4] - t * inv_s2);
 }
 
 // Per atom: the cube gather of Psi = psi + gE c h^3 phi and the sphere
 // gather of phi, combined into dL/dq and dL/dx.
 template <typename CT>
-__device__ __forceinline__ void adj_gather_atom(
-    const typename Vec4<CT>::type& a, int i, const Stencil<CT>& sp, const Stencil<CT>& sg,
-    double c, double gE_ch3, const CT* __restrict__ psi, const CT* __restrict__ phi,
-    const double* __restrict__ gfx, const double* __restrict__ gfy,
-    const double* __restrict__ gfz, double* __restrict__ dq, double* __restrict__ dx,
-    double* __restrict__ dy, double* __restrict__ dz) {
-  const int lane = threadIdx.x & 31;
-  const int W0 = 2 * sp.nst[0] + 1, W1 = 2 * sp.nst[1] + 1, W2 = 2 * sp.nst[2] + 1;
-  const double inv_s2 = 2.0 * (double)sp.inv_2s2;
-  {
-    const CT pos[3] = {a.x, a.y, a.z};
-    const double G[3] = {gfx ? gfx[i] : 0.0, gfy ? gfy[i] : 0.0, gfz ? gfz[i] : 0.0};
-    int c0[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) c0[d] = round_to_int(mul_rn(pos[d], sp.inv_h[d])) - sp.nst[d];
-    double P = 0, V[3] = {0, 0, 0}, T0 = 0, T1[3] = {0, 0, 0}, T2[3] = {0, 0, 0};
-    for (int t = lane; t < W0 * W1 * W2; t += 32) {
-      const int tz = t / (W0 * W1), r = t - tz * W0 * W1, ty = r / W0, tx = r - ty * W0;
-      const int p[3] = {c0[0] + tx, c0[1] + ty, c0[2] + tz};
-      CT u[3];
-#pragma unroll
-      for (int d = 0; d < 3; d++) u[d] = sub_rn(pos[d], mul_rn((CT)p[d], sp.h[d]));
-      const CT r2 = add_rn(add_rn(mul_rn(u[0], u[0]), mul_rn(u[1], u[1])), mul_rn(u[2], u[2]));
-      const long long idx = pmod(p[0], sp.M[0]) +
-                            ((long long)pmod(p[1], sp.M[1]) + (long long)pmod(p[2], sp.M[2]) * sp.M[1]) * sp.M[0];
-      const double e = (double)gexp(-r2 * sp.inv_2s2);
-      const double ph = (double)phi[idx];
-      const double Psi = (double)psi[idx] + gE_ch3 * ph;
-      const double g = (double)sp.pref * e * Psi;  // g(r - x) Psi
-      P += g;
-#pragma unroll
-      for (int d = 0; d < 3; d++) V[d] -= g * (double)u[d] * inv_s2;  // (r - x) = -u
-      if (r2 < sg.rcut2) {
-        const double t0 = e * ph;
-        const double Gu = G[0] * (double)u[0] + G[1] * (double)u[1] + G[2] * (double)u[2];
-        T0 += t0;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-          T1[d] += t0 * (double)u[d];
-          T2[d] += t0 * Gu * (double)u[d];
-        }
-      }
-    }
-    P = warp_sum(P);
-    T0 = warp_sum(T0);
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      V[d] = warp_sum(V[d]);
-      T1[d] = warp_sum(T1[d]);
-      T2[d] = warp_sum(T2[d]);
-    }
-    if (lane == 0) {
-      const double q = (double)a.w;
-      const double cA = c * (double)sg.pref;
-      dq[i] = P + cA * (G[0] * T1[0] + G[1] * T1[1] + G[2] * T1[2]);
-      dx[i] = q * V[0] + cA * q * (G[0] * T0 - T2[0] * inv_s2);
-      dy[i] = q * V[1] + cA * q * (G[1] * T0 - T2[1] * inv_s2);
-      dz[i] = q * V[2] + cA * q * (G[2] * T0 - T2[2] * inv_s2);
-    }
-  }
-}
-
-template <typename CT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * kAdjWarps)
     k_adj_gather(const typename Vec4<CT>::type* __restrict__ xyzq, const int* __restrict__ perm,
                  int n, Stencil<CT> sp /*spread*/, Stencil<CT> sg /*gather*/, double c,
                  double gE_ch3, const CT* __restrict__ psi, const CT* __restrict__ phi,
                  const double* __restrict__ gfx, const double* __restrict__ gfy,
                  const double* __restrict__ gfz, double* __restrict__ dq,
                  double* __restrict__ dx, double* __restrict__ dy, double* __restrict__ dz) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int ii = gw; ii < n; ii += nw)
-    adj_gather_atom<CT>(xyzq[ii], perm[ii], sp, sg, c, gE_ch3, psi, phi, gfx, gfy, gfz, dq, dx,
-                        dy, dz);
+  __shared__ AdjRowTab<CT> tabs[kAdjWarps];
+  __shared__ double sums[kAdjWarps][16];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  AdjRowTab<CT>& t = tabs[w];
+  for (int ii = blockIdx.x * kAdjWarps + w; ii < n; ii += gridDim.x * kAdjWarps) {
+    const auto a = xyzq[ii];
+    const int i = perm[ii];
+    const CT pos[3] = {a.x, a.y, a.z};
+    double G[3] = {0.0, 0.0, 0.0};
+    if (lane < 4 && gfx) {
+      G[0] = gfx[i];
+      G[1] = gfy[i];
+      G[2] = gfz[i];
+    }
+    const int c0x = adj_tables<CT>(pos, sp, t);
+    double v[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[k] = 0.0;
+    // a plane's sums over y at this lane's x offset: C over Psi, D over phi in the sphere
+    double C0 = 0, Cy = 0, D0 = 0, Dy = 0, Dyy = 0, ex = 0, ux = 0;
+    CT ux2 = 0, uz2 = 0;
+    CT lps[kAdjRows], lph[kAdjRows];
+    adj_planes<CT>(
+        pos, sp, t, c0x,
+        [&](int jz, CT e, CT u, CT u2) {
+          ex = (double)e;
+          ux = (double)u;
+          ux2 = u2;
+          uz2 = t.u2[1][jz];
+          C0 = Cy = D0 = Dy = Dyy = 0.0;
+        },
+        [&](int k, long long idx) {
+          lph[k] = phi[idx];
+          lps[k] = psi[idx];
+        },
+        [&](int k, int jy) {
+          const double ey = (double)t.e[0][jy], eu = (double)t.eu[0][jy];
+          const double ph = (double)lph[k], ps = fma(gE_ch3, ph, (double)lps[k]);
+          C0 = fma(ey, ps, C0);
+          Cy = fma(eu, ps, Cy);
+          if (add_rn(add_rn(ux2, t.u2[0][jy]), uz2) < sg.rcut2) {
+            D0 = fma(ey, ph, D0);
+            Dy = fma(eu, ph, Dy);
+            Dyy = fma(eu * (double)t.u[0][jy], ph, Dyy);
+          }
+        },
+        [&](int jz) {
+          const double f = ex * (double)t.e[1][jz], z = (double)t.u[1][jz];
+          const double a0 = f * C0, b0 = f * D0, by = f * Dy;
+          v[0] += a0;
+          v[1] = fma(a0, ux, v[1]);
+          v[2] = fma(f, Cy, v[2]);
+          v[3] = fma(a0, z, v[3]);
+          v[4] += b0;
+          v[5] = fma(b0, ux, v[5]);
+          v[6] += by;
+          v[7] = fma(b0, z, v[7]);
+          v[8] = fma(b0, ux * ux, v[8]);
+          v[9] = fma(by, ux, v[9]);
+          v[10] = fma(b0, ux * z, v[10]);
+          v[11] = fma(f, Dyy, v[11]);
+          v[12] = fma(by, z, v[12]);
+          v[13] = fma(b0, z * z, v[13]);
+        });
+    warp_sum16(v);
+    if (!(lane & 1)) sums[w][lane >> 1] = v[0];
+    __syncwarp();
+    if (lane < 4)
+      adj_outputs(sums[w], G, (double)a.w, (double)sp.pref, 2.0 * (double)sp.inv_2s2,
+                  c * (double)sg.pref, i, dq, dx, dy, dz);
+  }
 }
 
 // ===========================================================================
@@ -579,38 +680,15 @@ __device__ __forceinline__ void adj_gather_brick(
         Myz += a0 * uy * uz;
         Mzz += a0 * uz2;
       }
-      // the lanes' sums in FP64: at each step a lane keeps half of its values and
-      // hands the other half to its partner (the butterfly's sums, at a third of its
-      // shuffles); lane 2 i then holds value i, and the first four lanes form one
-      // output each
+      // lane 2 i then holds value i, and the first four lanes form one output each
       double v[16] = {P, Vx, Vy, Vz, T0, T1x, T1y, T1z, Mxx, Mxy, Mxz, Myy, Myz, Mzz, 0.0, 0.0};
-#pragma unroll
-      for (int h = 8; h > 0; h >>= 1) {
-        const bool up = lane & (2 * h);
-#pragma unroll
-        for (int i = 0; i < h; i++) {
-          const double give = up ? v[i] : v[i + h];
-          v[i] = (up ? v[i + h] : v[i]) + __shfl_xor_sync(0xffffffffu, give, 2 * h);
-        }
-      }
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      warp_sum16(v);
       double* m = reinterpret_cast<double*>(tb);  // the atom's tables are used up
       __syncwarp();
       if (!(lane & 1)) m[lane >> 1] = v[0];
       __syncwarp();
-      if (lane < 4) {
-        const double q64 = (double)a.w;
-        // lane 0: dL/dq from T1; lane 1 + d: dL/dx_d from row d of M
-        const int i0 = lane == 0 ? 5 : 7 + lane, i1 = lane == 0 ? 6 : lane == 1 ? 9 : 9 + lane,
-                  i2 = lane == 0 ? 7 : lane == 1 ? 10 : 10 + lane;
-        const double t = m[i0] * G[0] + m[i1] * G[1] + m[i2] * G[2];
-        const double Gd = lane == 1 ? G[0] : lane == 2 ? G[1] : G[2];
-        double* out = lane == 0 ? dq : lane == 1 ? dx : lane == 2 ? dy : dz;
-        // (r - x) = -u
-        out[o] = lane == 0 ? pref_sp * m[0] + cA * t
-                           : -q64 * pref_sp * inv_s2 * m[lane] +
-                                 cA * q64 * (Gd * m[4] - t * inv_s2);
-      }
+      if (lane < 4)
+        adj_outputs(m, G, (double)a.w, pref_sp, inv_s2, cA, o, dq, dx, dy, dz);
       __syncwarp();
     }
     __syncthreads();
@@ -966,7 +1044,7 @@ cudaError_t launch_adj_source(const typename Vec4<CT>::type* xyzq, const int* pe
                               const double* gfy, const double* gfz, CT* lambda, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int blocks = (int)std::min<long long>(sm_count() * 16, (n + 7) / 8);
-  k_adj_source<CT><<<blocks, 256, 0, st>>>(xyzq, perm, n, s, c, gfx, gfy, gfz, lambda);
+  k_adj_source<CT><<<blocks, 32 * kAdjWarps, 0, st>>>(xyzq, perm, n, s, c, gfx, gfy, gfz, lambda);
   return cudaGetLastError();
 }
 
@@ -978,7 +1056,7 @@ cudaError_t launch_adj_gather(const typename Vec4<CT>::type* xyzq, const int* pe
                               double* dy, double* dz, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int blocks = (int)std::min<long long>(sm_count() * 16, (n + 7) / 8);
-  k_adj_gather<CT><<<blocks, 256, 0, st>>>(xyzq, perm, n, sp, sg, c, gE_ch3, psi, phi, gfx, gfy,
+  k_adj_gather<CT><<<blocks, 32 * kAdjWarps, 0, st>>>(xyzq, perm, n, sp, sg, c, gE_ch3, psi, phi, gfx, gfy,
                                            gfz, dq, dx, dy, dz);
   return cudaGetLastError();
 }
