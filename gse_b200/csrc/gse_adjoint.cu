@@ -789,7 +789,7 @@ cudaError_t adj_scatter_w(const float4* sorted, const float4* gs, const int* sta
   k_adj_scatter<W><<<grd, kAdjScatterThreads, smem, st>>>(
       sorted, gs, start, b, s, (float)(c * (double)s.pref), nparts, grid64);
   e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || !lambda) return e;
   return launch_grid64_to_real(grid64, size, lambda, st);
 }
 

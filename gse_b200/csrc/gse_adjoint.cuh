@@ -10,7 +10,8 @@ namespace gse {
 
 // Tiled reverse pass of the mixed form (sorted atoms and bin starts as the
 // forward pass leaves them).  The source lambda is accumulated in `grid64`
-// (cleared here) and written as floats into `lambda`; gs: scratch [n].
+// (cleared here) and written as floats into `lambda` (NULL: left to the caller); gs:
+// scratch [n].
 cudaError_t launch_adj_scatter(const float4* sorted, const int* perm, int n, const int* start,
                                const BinLayout& b, const Stencil<float>& sg, double c,
                                const double* gfx, const double* gfy, const double* gfz,

@@ -569,6 +569,36 @@ bool make_green_callback_plan(gse_context_t* c) {
   return true;
 }
 
+// The own FFT solve of the mixed form: phi from the int64 grid (`fixed`) or the float
+// grid rho; rho_out (may be NULL) receives the float grid of the former, energy_out
+// the k-space energy.  From a scatter kernel directly before it on the stream the
+// forward pass may be launched as that kernel's dependent (pdl).
+gse_status_t own_solve(gse_context_t* c, bool fixed, float* rho_out, float* phi,
+                       double* energy_out, bool pdl) {
+  const int M = c->p.size_x;
+  {
+    StageTimer tm(c, GSE_STAGE_FFT_FORWARD);
+    c->launches += 1;
+    CU(launch_own_fft_xy_forward(M, fixed ? c->d_fixed : nullptr,
+                                 fixed ? nullptr : (const float*)c->d_rho,
+                                 std::exp2(-(double)kFlushBits), rho_out, (float2*)c->d_rhok,
+                                 c->d_fft_tw, c->bl.flags, pdl, c->fft_stall_test, c->stream));
+  }
+  {
+    StageTimer tm(c, GSE_STAGE_GREEN);
+    c->launches += 1;
+    CU(launch_own_fft_z_green(M, (float2*)c->d_rhok, (const float*)c->d_gtab, c->d_fft_tw,
+                              c->d_partials,
+                              reinterpret_cast<unsigned*>(c->d_partials + kEnergyPartials),
+                              energy_factor(c), energy_out, !c->timing, c->stream));
+  }
+  StageTimer tm(c, GSE_STAGE_FFT_BACKWARD);
+  c->launches += 1;
+  CU(launch_own_fft_xy_inverse(M, (const float2*)c->d_rhok, phi, c->d_fft_tw, c->bl.flags,
+                               !c->timing, c->stream));
+  return GSE_OK;
+}
+
 gse_status_t do_solve_ctx(gse_context_t* c) {
   const GreenGeom g = green_geom(c, c->sigma2, c->p.box_x, c->p.box_y, c->p.box_z, true);
   if (!c->d_gtab) CU(cudaMalloc(&c->d_gtab, c->ksize * c->ct));  // fixed address from here on
@@ -579,32 +609,13 @@ gse_status_t do_solve_ctx(gse_context_t* c) {
       CU(launch_green_table<float>(g, (float*)c->d_gtab, c->stream));
       c->gtab_valid = true;
     }
-    const int M = c->p.size_x;
-    {
-      StageTimer tm(c, GSE_STAGE_FFT_FORWARD);
-      c->launches += 1;
-      const bool fx = c->fixed_pending;
-      // from a deferred spread (forward_body) the solve follows the spread
-      // kernel directly, and each pass follows the previous one: dependent
-      // launches, unless stage timing puts events between them
-      CU(launch_own_fft_xy_forward(M, fx ? c->d_fixed : nullptr, fx ? nullptr : (float*)c->d_rho,
-                                   std::exp2(-(double)kFlushBits), fx ? (float*)c->d_rho : nullptr,
-                                   (float2*)c->d_rhok, c->d_fft_tw, c->bl.flags,
-                                   fx && !c->timing, c->fft_stall_test, c->stream));
-      c->fixed_pending = false;
-    }
-    {
-      StageTimer tm(c, GSE_STAGE_GREEN);
-      c->launches += 1;
-      CU(launch_own_fft_z_green(M, (float2*)c->d_rhok, (const float*)c->d_gtab, c->d_fft_tw,
-                                c->d_partials,
-                                reinterpret_cast<unsigned*>(c->d_partials + kEnergyPartials),
-                                energy_factor(c), c->d_scalars, !c->timing, c->stream));
-    }
-    StageTimer tm(c, GSE_STAGE_FFT_BACKWARD);
-    c->launches += 1;
-    CU(launch_own_fft_xy_inverse(M, (const float2*)c->d_rhok, (float*)c->d_phi, c->d_fft_tw,
-                                 c->bl.flags, !c->timing, c->stream));
+    const bool fx = c->fixed_pending;
+    // from a deferred spread (forward_body) the solve follows the spread
+    // kernel directly, and each pass follows the previous one: dependent
+    // launches, unless stage timing puts events between them
+    TRY(own_solve(c, fx, fx ? (float*)c->d_rho : nullptr, (float*)c->d_phi, c->d_scalars,
+                  fx && !c->timing));
+    c->fixed_pending = false;
     return GSE_OK;
   }
   if (!c->green_cb_tried && c->size >= kGreenCallbackMinPoints) {
@@ -1687,16 +1698,17 @@ gse_status_t gse_adjoint(gse_context_t* c, int n, const void* xyzq, double dLdE,
   const double h3 = (c->p.box_x / c->p.size_x) * (c->p.box_y / c->p.size_y) *
                     (c->p.box_z / c->p.size_z);
   const double gE_ch3 = dLdE * c->p.ccelec * h3;
-  // forward grids, recomputed from the inputs (rho -> phi)
-  if (c->fp64)
+  // forward grids, recomputed from the inputs (rho -> phi), as forward_body does
+  if (c->fp64) {
     TRY(bin_atoms<double>(c, n, dxq, stencil_of<double>(c, box.v, c->sigma1, c->rcut1, false, false),
                           false, true));
-  else
-    TRY(bin_atoms<float>(c, n, dxq, stencil_of<float>(c, box.v, c->sigma1, c->rcut1, false, false)));
-  if (c->fp64)
     TRY(do_spread<double>(c, n, dxq, box.v, c->sigma1, c->rcut1, false, true));
-  else
-    TRY(do_spread<float>(c, n, dxq, box.v, c->sigma1, c->rcut1, false, true));
+  } else {
+    const Stencil<float> s = stencil_of<float>(c, box.v, c->sigma1, c->rcut1, false, false);
+    const bool zeroed = !c->timing && tiled_ok<float>(c, s);
+    TRY(bin_atoms<float>(c, n, dxq, s, zeroed));
+    TRY(do_spread<float>(c, n, dxq, box.v, c->sigma1, c->rcut1, false, true, true, zeroed));
+  }
   TRY(do_solve_ctx(c));
   c->phi_valid = true;
   c->energy_valid = true;
@@ -1705,10 +1717,10 @@ gse_status_t gse_adjoint(gse_context_t* c, int n, const void* xyzq, double dLdE,
       !c->fp64 && tiled_ok<float>(c, stencil_of<float>(c, box.v, c->sigma1, c->rcut1, true, false));
   if (tiled_mixed) {
     const Stencil<float> sg = stencil_of<float>(c, box.v, c->sigma1, c->rcut1, true, false);
-    c->launches += 3;
+    c->launches += c->own_fft ? 2 : 3;
     CU(launch_adj_scatter((const float4*)c->d_sorted, c->d_perm, n, c->d_bstart, c->bl, sg,
                           c->p.ccelec, gd[0], gd[1], gd[2], (float4*)(c->d_adj + 7 * cap),
-                          c->d_fixed, (float*)c->d_rho, c->stream));
+                          c->d_fixed, c->own_fft ? nullptr : (float*)c->d_rho, c->stream));
   } else {
   CU(cudaMemsetAsync(c->d_rho, 0, c->size * c->ct, c->stream));
   c->launches += 3;
@@ -1722,7 +1734,11 @@ gse_status_t gse_adjoint(gse_context_t* c, int n, const void* xyzq, double dLdE,
                                 gd[1], gd[2], (float*)c->d_rho, c->stream));
   }
   }
-  TRY(do_solve(c, c->d_rho, c->d_rho, c->sigma2, c->p.box_x, c->p.box_y, c->p.box_z, false));
+  // (the own FFT reads the int64 grid; its k-space sum of lambda goes to a scratch slot)
+  if (tiled_mixed && c->own_fft)
+    TRY(own_solve(c, true, nullptr, (float*)c->d_rho, c->d_scalars + 1, false));
+  else
+    TRY(do_solve(c, c->d_rho, c->d_rho, c->sigma2, c->p.box_x, c->p.box_y, c->p.box_z, false));
   c->rho_valid = false;
   const bool dev_out = is_device_ptr(dq) && is_device_ptr(dx) && is_device_ptr(dy) &&
                        is_device_ptr(dz);
