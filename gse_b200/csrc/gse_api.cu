@@ -161,7 +161,7 @@ struct gse_context {
   double* d_basis = nullptr;  // FP64 form: spread weights' basis of the sorted atoms
   int* d_bcounts = nullptr;
   int* d_bstart = nullptr;
-  int* d_blstart = nullptr;  // mixed form: tile-local bin starts of the scan
+  int* d_blstart = nullptr;  // tile-local bin starts of the scan
   int* d_btiles = nullptr;
   // Green's function table of the context's own solve (sigma2, box)
   void* d_gtab = nullptr;
@@ -391,23 +391,19 @@ gse_status_t bin_atoms(gse_context_t* c, int n, const void* dx, const Stencil<CT
                        bool clear_fixed = false, bool basis = false) {
   typedef typename Vec4<CT>::type V;
   StageTimer tm(c, GSE_STAGE_BIN);
-  BinScratch w{c->d_bkey, c->d_bcounts, c->d_bstart, c->d_btiles, c->d_btmp, c->d_badmap};
-  // mixed: count, a tile-local scan and the placement that applies the tile
-  // offsets (the counts stay zero between calls); FP64: count, three scan
-  // passes and a stable placement in two kernels
-  if (!c->fp64) {
-    w.lstart = c->d_blstart;
-    w.counts_zero = true;
-    if (clear_fixed) {
-      w.clear = c->d_fixed;
-      w.clear_n = c->size;
-    }
+  BinScratch w{c->d_bkey, c->d_bcounts, c->d_bstart, c->d_btiles,
+               c->d_btmp, c->d_blstart, c->d_badmap};
+  // count, a tile-local scan, the placement that applies the tile offsets, and in the
+  // FP64 form the stable order within the bins
+  if (!c->fp64 && clear_fixed) {
+    w.clear = c->d_fixed;
+    w.clear_n = c->size;
   }
   if constexpr (sizeof(CT) == 8) {
     if (basis && tiled_ok<CT>(c, s))
       w.basis = SpreadBasis{{s.h[0], s.h[1], s.h[2]}, s.inv_2s2, s.pref, s.nst[0], c->d_basis};
   }
-  c->launches += c->fp64 ? (n > 0 ? 6 : 3) : (n > 0 ? 3 : 2);
+  c->launches += n > 0 ? (c->fp64 ? 4 : 3) : 2;
   CU(launch_bin_sorted<CT>((const V*)dx, n, c->bl, s.inv_h[0], s.inv_h[1], s.inv_h[2], w,
                            (V*)c->d_sorted, c->d_perm, c->stream));
   return GSE_OK;
@@ -936,7 +932,7 @@ gse_status_t gse_create(const gse_params_t* params, gse_context_t** out) {
   c->nbins2 = bin_count(c->bl);
   CUC(cudaMalloc(&c->d_bcounts, sizeof(int) * c->nbins2));
   CUC(cudaMemset(c->d_bcounts, 0, sizeof(int) * c->nbins2));
-  if (!c->fp64) CUC(cudaMalloc(&c->d_blstart, sizeof(int) * c->nbins2));
+  CUC(cudaMalloc(&c->d_blstart, sizeof(int) * c->nbins2));
   CUC(cudaMalloc(&c->d_bstart, sizeof(int) * (c->nbins2 + 1)));
   CUC(cudaMalloc(&c->d_btiles, sizeof(int) * (c->nbins2 / 4096 + 2)));
   CUC(cudaMalloc(&c->d_partials, sizeof(double) * (kEnergyPartials + 1)));
@@ -946,6 +942,8 @@ gse_status_t gse_create(const gse_params_t* params, gse_context_t** out) {
   CUC(cudaMemset(c->d_bad, 0, sizeof(int)));
   CUC(cudaMemset(c->d_scalars, 0, sizeof(double) * 16));
   CUC(cudaMallocHost(&c->h_pinned, sizeof(double) * 4));
+  // the bin counts must be zero before a first call on a non-blocking stream
+  CUC(cudaStreamSynchronize(nullptr));
   {
     int* hb = nullptr;
     CUC(cudaHostAlloc(&hb, sizeof(int), cudaHostAllocMapped));
@@ -1973,7 +1971,7 @@ gse_status_t gse_ewald_direct(int device, void* stream, double sigma, double rcu
   const EwdGeom g = ewald_direct_geom(sigma, rcut, box, ccelec);
   const int ntiles = (g.ncell + 4095) / 4096;
   // one allocation: ints, then doubles (8-byte aligned), then atoms
-  const size_t n_int = 2 * (size_t)n + (size_t)g.ncell * 2 + 1 + ntiles + n + 1 + ex_idx.size() +
+  const size_t n_int = 2 * (size_t)n + (size_t)g.ncell * 3 + 1 + ntiles + n + 1 + ex_idx.size() +
                        (ex_start.empty() ? 0 : n + 1);
   const size_t off_d = (n_int * sizeof(int) + 31) / 32 * 32;
   const size_t n_part = (size_t)g.ncell * ewald_direct_split(n, g);
@@ -2011,6 +2009,8 @@ gse_status_t gse_ewald_direct(int device, void* stream, double sigma, double rcu
   ip += g.ncell + 1;
   w.tile_sums = ip;
   ip += ntiles;
+  w.lstart = ip;
+  ip += g.ncell;
   w.perm = ip;
   ip += n;
   w.done = (unsigned*)ip;

@@ -73,6 +73,7 @@ struct gse_batch {
   int* d_counts = nullptr;
   int* d_start = nullptr;
   int* d_tiles = nullptr;
+  int* d_lstart = nullptr;
   long long* d_g64 = nullptr;
   float* d_rho = nullptr;
   float* d_phi = nullptr;
@@ -216,7 +217,8 @@ BatchFused fused_args(const gse_batch_t* b) {
   a.nbins = b->nbins;
   a.sys = b->d_sys;
   a.first = b->d_first;
-  a.w = BinScratch{b->d_key, b->d_counts, b->d_start, b->d_tiles, b->d_tmp};
+  a.w = BinScratch{b->d_key, b->d_counts, b->d_start,
+                   b->d_tiles, b->d_tmp, b->d_lstart};
   a.sorted = b->d_sorted;
   a.perm = b->d_perm;
   a.scat = b->d_scat;
@@ -261,7 +263,8 @@ gse_status_t run_forward(gse_batch_t* b) {
     BCU(launch_batch_forward_fused(fused_args(b), b->fused_ctas, b->gather_lanes, st));
     return GSE_OK;
   }
-  BinScratch w{b->d_key, b->d_counts, b->d_start, b->d_tiles, b->d_tmp};
+  BinScratch w{b->d_key, b->d_counts, b->d_start,
+                   b->d_tiles, b->d_tmp, b->d_lstart};
   BCU(launch_batch_bin(b->d_xyzq, b->ntot, b->d_sys, b->d_first, b->nsys, b->nbins, w,
                        b->d_sorted, b->d_perm, st));
   BCU(launch_batch_spread(b->d_sorted, b->d_start, b->d_sys, b->d_scat, b->scat_seg.data(),
@@ -460,7 +463,9 @@ gse_status_t gse_batch_create(const gse_params_t* common, int nsys, const gse_sy
   BCUC(cudaMalloc(&b->d_key, sizeof(int) * na));
   BCUC(cudaMalloc(&b->d_tmp, sizeof(int) * na));
   BCUC(cudaMalloc(&b->d_counts, sizeof(int) * b->nbins));
+  BCUC(cudaMemset(b->d_counts, 0, sizeof(int) * b->nbins));
   BCUC(cudaMalloc(&b->d_start, sizeof(int) * (b->nbins + 1)));
+  BCUC(cudaMalloc(&b->d_lstart, sizeof(int) * b->nbins));
   BCUC(cudaMalloc(&b->d_tiles, sizeof(int) * (b->nbins / 4096 + 2)));
   BCUC(cudaMalloc(&b->d_g64, sizeof(long long) * b->gtot));
   BCUC(cudaMalloc(&b->d_rho, sizeof(float) * b->gtot));
@@ -561,7 +566,7 @@ gse_status_t gse_batch_destroy(gse_batch_t* b) {
   void* ptrs[] = {b->d_line_first, b->d_epart, b->d_qctr,
                   b->d_sys, b->d_first, b->d_kfirst, b->d_ksys, b->d_scat, b->d_gath, b->d_agath,
                   b->d_xyzq, b->d_sorted, b->d_perm, b->d_key, b->d_tmp, b->d_counts,
-                  b->d_start, b->d_tiles, b->d_g64, b->d_rho, b->d_phi, b->d_lam,
+                  b->d_start, b->d_tiles, b->d_lstart, b->d_g64, b->d_rho, b->d_phi, b->d_lam,
                   b->d_rhok, b->d_gtab, b->d_energy, b->d_dLdE, b->d_forces, b->d_gin, b->d_gs,
                   b->d_gout};
   for (void* q : ptrs) cudaFree(q);

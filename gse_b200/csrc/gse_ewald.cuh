@@ -56,6 +56,7 @@ struct EwdScratch {
   int* counts;      // [ncell]
   int* start;       // [ncell + 1]
   int* tile_sums;   // [ceil(ncell / 4096)]
+  int* lstart;      // [ncell]
   int* tmp;         // [n]
   double4* sorted;  // [n] atoms in cell order
   int* perm;        // [n] original index of each sorted atom

@@ -50,7 +50,9 @@ __device__ __forceinline__ int ewd_cell_axis(double x, double box, double inv_bo
 }
 
 __global__ void k_ewd_cell_count(const double4* __restrict__ xyzq, int n, EwdGeom g,
-                                 int* __restrict__ key, int* __restrict__ counts) {
+                                 int* __restrict__ key, int* __restrict__ counts,
+                                 int* __restrict__ rank) {
+  pdl_trigger();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double4 p = xyzq[i];
     const int cx = ewd_cell_axis(p.x, g.box[0], g.inv_box[0], g.nc[0]);
@@ -58,7 +60,7 @@ __global__ void k_ewd_cell_count(const double4* __restrict__ xyzq, int n, EwdGeo
     const int cz = ewd_cell_axis(p.z, g.box[2], g.inv_box[2], g.nc[2]);
     const int k = cx + g.nc[0] * (cy + g.nc[1] * cz);
     key[i] = k;
-    atomicAdd(&counts[k], 1);
+    rank[i] = atomicAdd(&counts[k], 1);
   }
 }
 
@@ -277,13 +279,14 @@ cudaError_t launch_ewald_direct(const double4* xyzq, int n, const EwdGeom& g, Ew
   e = cudaMemsetAsync(w.done, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
   const int gb = n > 0 ? (int)std::min<long long>(sm_count() * 8, (n + 255) / 256) : 1;
-  if (n > 0) k_ewd_cell_count<<<gb, 256, 0, st>>>(xyzq, n, g, w.key, w.counts);
-  BinScratch b;
+  if (n > 0) k_ewd_cell_count<<<gb, 256, 0, st>>>(xyzq, n, g, w.key, w.counts, w.perm);
+  BinScratch b = {};
   b.key = w.key;
   b.counts = w.counts;
   b.start = w.start;
   b.tile_sums = w.tile_sums;
   b.tmp = w.tmp;
+  b.lstart = w.lstart;
   e = launch_bin_scan_place<double>(xyzq, n, g.ncell, b, w.sorted, w.perm, st);
   if (e != cudaSuccess) return e;
   const size_t smem = kEwdTile * (4 * sizeof(double) + sizeof(int));

@@ -52,17 +52,12 @@ struct SpreadBasis {
 
 struct BinScratch {
   int* key;        // [n]
-  int* counts;     // [nbins]
+  int* counts;     // [nbins], zero on entry and again after the placement
   int* start;      // [nbins + 1]
   int* tile_sums;  // [ceil(nbins / 4096)]
-  int* tmp;        // [n]: the FP64 stable placement's scratch; the mixed form's ranks in bin
+  int* tmp;        // [n]: the mixed form's ranks in bin; the FP64 form's unordered placement
+  int* lstart;     // [nbins]: the scan's tile-local prefix
   int* bad = nullptr;   // set to 1 when a position or charge is not finite (may be NULL)
-  // mixed form: the scan's tile-local prefix [nbins] (the placement applies the tile
-  // offsets and writes `start`); NULL: a three-kernel scan writes `start` directly
-  int* lstart = nullptr;
-  // mixed form: `counts` are zero on entry (the order-free placement counts every
-  // bin back down to zero), so the binning does not clear them
-  bool counts_zero = false;
   // an int64 array of clear_n elements (16-byte aligned) that the counting
   // kernel clears on the way (the mixed form's spread grid); NULL: none
   long long* clear = nullptr;
@@ -70,6 +65,13 @@ struct BinScratch {
   // FP64 form: weights' basis of the sorted atoms, for the spread that follows
   SpreadBasis basis = {};
 };
+
+// Where the counting kernel leaves each atom's rank in its bin: the FP64 form's perm
+// is written after the ranks are read, its tmp before.
+template <typename CT>
+inline int* bin_rank(const BinScratch& w, int* perm) {
+  return sizeof(CT) == 8 ? perm : w.tmp;
+}
 
 inline BinLayout make_bin_layout(const int M[3], int bin_width) {
   BinLayout b;
