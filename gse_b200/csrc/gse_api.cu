@@ -403,7 +403,7 @@ gse_status_t bin_atoms(gse_context_t* c, int n, const void* dx, const Stencil<CT
     if (basis && tiled_ok<CT>(c, s))
       w.basis = SpreadBasis{{s.h[0], s.h[1], s.h[2]}, s.inv_2s2, s.pref, s.nst[0], c->d_basis};
   }
-  c->launches += n > 0 ? (c->fp64 ? 4 : 3) : 2;
+  c->launches += bin_small(c->fp64, n, c->nbins2) ? 1 : n > 0 ? (c->fp64 ? 4 : 3) : 2;
   CU(launch_bin_sorted<CT>((const V*)dx, n, c->bl, s.inv_h[0], s.inv_h[1], s.inv_h[2], w,
                            (V*)c->d_sorted, c->d_perm, c->stream));
   return GSE_OK;

@@ -28,6 +28,18 @@ namespace gse {
 // ===========================================================================
 // Binning
 // ===========================================================================
+template <typename V>
+__device__ __forceinline__ int bin_of(const V& a, const BinLayout& b, decltype(V::x) inv_hx,
+                                      decltype(V::x) inv_hy, decltype(V::x) inv_hz,
+                                      int* __restrict__ bad) {
+  if (bad && !(isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w)))
+    *bad = kFlagNonFinite;  // the bin below is still in range (wrap1 of any int)
+  const int cx = wrap1(centre_cell(a.x, inv_hx), b.M[0]);
+  const int cy = wrap1(centre_cell(a.y, inv_hy), b.M[1]);
+  const int cz = wrap1(centre_cell(a.z, inv_hz), b.M[2]);
+  return (cz * b.M[1] + cy) * b.nbx + (cx >> b.bxs);
+}
+
 template <typename CT>
 __global__ void k_bin_count(const typename Vec4<CT>::type* __restrict__ xyzq, int n, BinLayout b,
                             CT inv_hx, CT inv_hy, CT inv_hz, int* __restrict__ key,
@@ -42,13 +54,7 @@ __global__ void k_bin_count(const typename Vec4<CT>::type* __restrict__ xyzq, in
     if ((clear_n & 1) && first == 0) clear[clear_n - 1] = 0;
   }
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const auto a = xyzq[i];
-    if (bad && !(isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w)))
-      *bad = kFlagNonFinite;  // the bin below is still in range (wrap1 of any int)
-    const int cx = wrap1(centre_cell(a.x, inv_hx), b.M[0]);
-    const int cy = wrap1(centre_cell(a.y, inv_hy), b.M[1]);
-    const int cz = wrap1(centre_cell(a.z, inv_hz), b.M[2]);
-    const int k = (cz * b.M[1] + cy) * b.nbx + (cx >> b.bxs);
+    const int k = bin_of(xyzq[i], b, inv_hx, inv_hy, inv_hz, bad);
     key[i] = k;
     // the atom's place among its bin's atoms (in counting order), so the placement
     // needs no atomics
@@ -131,6 +137,29 @@ __global__ void __launch_bounds__(256)
   if (gtid == 0) start[nb] = off[ntiles - 1] + tile_sums[ntiles - 1];
 }
 
+// The spread weights' basis of atom `a` into slot `slot` of sb.out.
+__device__ __forceinline__ void store_basis(const double4& a, int slot, const BinLayout& b,
+                                            const double3& inv_h, const SpreadBasis& sb) {
+  const double x[3] = {a.x, a.y, a.z}, ih[3] = {inv_h.x, inv_h.y, inv_h.z};
+  double v[kBasis64];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const int c = centre_cell(x[d], ih[d]);
+    // offset of the centre point, from the first point's offset as the reference
+    // rounds it (d0 = (c - n) h - x, CpuGaussCharge.cpp:311-329)
+    const double h = sb.h[d], hh = h * h;
+    const double dc = sub_rn(mul_rn((double)(c - sb.nst), h), x[d]) + (double)sb.nst * h;
+    const double wc = exp(mul_rn(mul_rn(-dc, dc), sb.inv_2s2));
+    v[3 * d] = d == 0 ? a.w * sb.pref * wc : wc;
+    v[3 * d + 1] = exp(-(2 * dc * h + hh) * sb.inv_2s2);
+    v[3 * d + 2] = exp(-(hh - 2 * dc * h) * sb.inv_2s2);
+    if (d == 0) v[9] = (double)wrap1(c, b.M[0]);
+  }
+  double2* o = reinterpret_cast<double2*>(sb.out + (long long)slot * kBasis64);
+#pragma unroll
+  for (int k = 0; k < kBasis64 / 2; k++) o[k] = make_double2(v[2 * k], v[2 * k + 1]);
+}
+
 // Stable placement (FP64 form): an atom's rank in its bin is the number of bin
 // members (tmp, in any order) with a smaller original index.
 __global__ void k_bin_place_stable(const double4* __restrict__ xyzq, int n,
@@ -147,25 +176,69 @@ __global__ void k_bin_place_stable(const double4* __restrict__ xyzq, int n,
     const double4 a = xyzq[i];
     sorted[s + r] = a;
     perm[s + r] = i;
-    if (sb.out) {
-      const double x[3] = {a.x, a.y, a.z}, ih[3] = {inv_h.x, inv_h.y, inv_h.z};
-      double v[kBasis64];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const int c = centre_cell(x[d], ih[d]);
-        // offset of the centre point, from the first point's offset as the reference
-        // rounds it (d0 = (c - n) h - x, CpuGaussCharge.cpp:311-329)
-        const double h = sb.h[d], hh = h * h;
-        const double dc = sub_rn(mul_rn((double)(c - sb.nst), h), x[d]) + (double)sb.nst * h;
-        const double wc = exp(mul_rn(mul_rn(-dc, dc), sb.inv_2s2));
-        v[3 * d] = d == 0 ? a.w * sb.pref * wc : wc;
-        v[3 * d + 1] = exp(-(2 * dc * h + hh) * sb.inv_2s2);
-        v[3 * d + 2] = exp(-(hh - 2 * dc * h) * sb.inv_2s2);
-        if (d == 0) v[9] = (double)wrap1(c, b.M[0]);
-      }
-      double2* o = reinterpret_cast<double2*>(sb.out + (long long)(s + r) * kBasis64);
-#pragma unroll
-      for (int k = 0; k < kBasis64 / 2; k++) o[k] = make_double2(v[2 * k], v[2 * k + 1]);
+    if (sb.out) store_basis(a, s + r, b, inv_h, sb);
+  }
+}
+
+// The whole binning of few atoms in one launch (bin_small): block 0, an atom per
+// thread, counts, scans and places them with the bins in shared memory (nb ints);
+// the other blocks clear the mixed form's grid.  The result is that of the kernels
+// above; their global counts stay zero.
+template <typename CT>
+__global__ void __launch_bounds__(kBinSmall)
+    k_bin_small(const typename Vec4<CT>::type* __restrict__ xyzq, int n, BinLayout b, CT inv_hx,
+                CT inv_hy, CT inv_hz, int nb, typename Vec4<CT>::type* __restrict__ sorted,
+                int* __restrict__ perm, int* __restrict__ start, int* __restrict__ bad,
+                long long* __restrict__ clear, long long clear_n, SpreadBasis sb) {
+  pdl_trigger();
+  const int tid = threadIdx.x;
+  if (blockIdx.x > 0) {
+    for (long long i = (blockIdx.x - 1) * (long long)kBinSmall + tid; i < clear_n;
+         i += (gridDim.x - 1) * (long long)kBinSmall)
+      clear[i] = 0;
+    return;
+  }
+  extern __shared__ int bins[];  // [nb] counts, then starts
+  __shared__ int tmp[kBinSmall];
+  typename Vec4<CT>::type a = {};
+  if (tid < n) a = xyzq[tid];
+  for (int i = tid; i < nb; i += kBinSmall) bins[i] = 0;
+  __syncthreads();
+  int k = 0, r = 0;
+  if (tid < n) {
+    k = bin_of(a, b, inv_hx, inv_hy, inv_hz, bad);
+    r = atomicAdd(&bins[k], 1);
+  }
+  __syncthreads();
+  const int per = (nb + kBinSmall - 1) / kBinSmall, i0 = min(tid * per, nb),
+            i1 = min(i0 + per, nb);
+  int s = 0;
+  for (int i = i0; i < i1; i++) s += bins[i];
+  int run = block_exclusive_scan(s, nullptr);
+  for (int i = i0; i < i1; i++) {
+    const int c = bins[i];
+    bins[i] = run;
+    run += c;
+  }
+  __syncthreads();
+  if (tid < n) {
+    r += bins[k];
+    if (sizeof(CT) == 8) tmp[r] = tid;
+  }
+  for (int i = tid; i <= nb; i += kBinSmall) start[i] = i < nb ? bins[i] : n;
+  if constexpr (sizeof(CT) == 8) {
+    __syncthreads();
+    if (tid < n) {
+      r = bins[k];
+      const int e = k + 1 < nb ? bins[k + 1] : n;
+      for (int j = bins[k]; j < e; j++) r += (tmp[j] < tid);
+    }
+  }
+  if (tid < n) {
+    sorted[r] = a;
+    perm[r] = tid;
+    if constexpr (sizeof(CT) == 8) {
+      if (sb.out) store_basis(a, r, b, make_double3(inv_hx, inv_hy, inv_hz), sb);
     }
   }
 }
@@ -629,6 +702,14 @@ cudaError_t launch_bin_sorted(const typename Vec4<CT>::type* xyzq, int n, const 
   const int nb = b.M[1] * b.M[2] * b.nbx;
   const int ntiles = (nb + kScanTile - 1) / kScanTile;
   if (ntiles > kScanTile) return cudaErrorInvalidValue;
+  if (bin_small(sizeof(CT) == 8, n, nb)) {
+    const int nclear =
+        w.clear ? (int)std::min<long long>(sm_count(), (w.clear_n + kBinSmall - 1) / kBinSmall) : 0;
+    k_bin_small<CT><<<1 + nclear, kBinSmall, sizeof(int) * nb, st>>>(
+        xyzq, n, b, inv_hx, inv_hy, inv_hz, nb, sorted, perm, w.start, w.bad, w.clear, w.clear_n,
+        w.basis);
+    return cudaGetLastError();
+  }
   cudaError_t e = cudaSuccess;
   // a grid to clear takes every SM; the atoms alone, one thread each up to that
   const int gb = w.clear ? sm_count() * 8
