@@ -73,14 +73,13 @@ def algorithmic_flops(stage: str) -> float:
     raise ValueError(stage)
 
 
-# what limits each kernel, from the committed full ncu capture of the
-# benchmark workload (profiles/spread_gather_water262k_mixed_full.md)
+# what limits each kernel, from the committed ncu counters of the
+# benchmark workload (profiles/spread_gather_water262k_mixed_counters.md)
 LIMITER = {
-    "gather": "latency and instruction issue at low occupancy (ncu: 500 warp instructions "
-              "per atom, 64% issue-active, 16 warps per SM); FP32 lanes are the arithmetic "
-              "roofline",
-    "spread": "shared-memory integer reductions and instruction issue (ncu: 424 warp "
-              "instructions per atom, 74% issue-active, LSU pipe 72% busy)",
+    "gather": "instruction issue and latency (ncu: 510 warp instructions per atom, 75% "
+              "issue-active, 23 warps per SM); FP32 lanes are the arithmetic roofline",
+    "spread": "shared-memory integer reductions and instruction issue (ncu: 428 warp "
+              "instructions per atom, 76% issue-active, LSU pipe 67% busy)",
 }
 
 
