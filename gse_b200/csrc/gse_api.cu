@@ -163,9 +163,10 @@ struct gse_context {
   int* d_bstart = nullptr;
   int* d_blstart = nullptr;  // tile-local bin starts of the scan
   int* d_btiles = nullptr;
-  // Green's function table of the context's own solve (sigma2, box)
+  // Green's function table of the context's own solve (sigma2, box) and the box that
+  // it was formed for (zeros: none yet)
   void* d_gtab = nullptr;
-  bool gtab_valid = false;
+  double gtab_box[3] = {0, 0, 0};
   // adjoint staging: upstream force gradients (3 x cap) and outputs (4 x cap)
   double* d_adj = nullptr;
   size_t adj_cap = 0;
@@ -595,16 +596,32 @@ gse_status_t own_solve(gse_context_t* c, bool fixed, float* rho_out, float* phi,
   return GSE_OK;
 }
 
-gse_status_t do_solve_ctx(gse_context_t* c) {
+// The table holds the Green's function of the context's present box.
+bool gtab_current(const gse_context_t* c) {
+  return c->gtab_box[0] == c->p.box_x && c->gtab_box[1] == c->p.box_y &&
+         c->gtab_box[2] == c->p.box_z;
+}
+
+gse_status_t ensure_gtab(gse_context_t* c) {
+  if (gtab_current(c)) return GSE_OK;
   const GreenGeom g = green_geom(c, c->sigma2, c->p.box_x, c->p.box_y, c->p.box_z, true);
   if (!c->d_gtab) CU(cudaMalloc(&c->d_gtab, c->ksize * c->ct));  // fixed address from here on
+  if (c->fp64)
+    CU(launch_green_table<double>(g, (double*)c->d_gtab, c->stream));
+  else
+    CU(launch_green_table<float>(g, (float*)c->d_gtab, c->stream));
+  c->gtab_box[0] = c->p.box_x;
+  c->gtab_box[1] = c->p.box_y;
+  c->gtab_box[2] = c->p.box_z;
+  return GSE_OK;
+}
+
+gse_status_t do_solve_ctx(gse_context_t* c) {
+  TRY(ensure_gtab(c));  // before the callback plan, which keeps the table's address
+  const GreenGeom g = green_geom(c, c->sigma2, c->p.box_x, c->p.box_y, c->p.box_z, true);
   if (c->own_fft) {
     // mixed form, cubic M = 16 N2: three passes of this library's own FFT;
     // the Green's multiply and the k-space energy sit in the z pass
-    if (!c->gtab_valid) {
-      CU(launch_green_table<float>(g, (float*)c->d_gtab, c->stream));
-      c->gtab_valid = true;
-    }
     const bool fx = c->fixed_pending;
     // from a deferred spread (forward_body) the solve follows the spread
     // kernel directly, and each pass follows the previous one: dependent
@@ -622,13 +639,6 @@ gse_status_t do_solve_ctx(gse_context_t* c) {
       c->green_cb_tried = true;
     }
     cudaGetLastError();
-  }
-  if (!c->gtab_valid) {
-    if (c->fp64)
-      CU(launch_green_table<double>(g, (double*)c->d_gtab, c->stream));
-    else
-      CU(launch_green_table<float>(g, (float*)c->d_gtab, c->stream));
-    c->gtab_valid = true;
   }
   {
     StageTimer tm(c, GSE_STAGE_FFT_FORWARD);
@@ -1026,7 +1036,6 @@ gse_status_t gse_set_box(gse_context_t* c, double bx, double by, double bz) {
     return s;
   }
   c->phi_valid = c->energy_valid = false;
-  c->gtab_valid = false;
   return GSE_OK;
 }
 
@@ -1173,6 +1182,9 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
       he = energy && !is_device_ptr(energy);
     }
     if ((he ? reinterpret_cast<double*>(uintptr_t(1)) : energy) == k.e) {
+      // the graph reads the table, which another call may have formed for another
+      // box since
+      TRY(ensure_gtab(c));
       CU(cudaGraphLaunch(c->fwd_exec, c->stream));
       c->fwd_replays++;
       c->launches += c->fwd_launches;
@@ -1199,7 +1211,7 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
   const bool host_io = host_e || (fx && !is_device_ptr(fx)) || (fy && !is_device_ptr(fy)) ||
                        (fz && !is_device_ptr(fz));
   const bool graphable = c->fwd_graphs && !c->timing && n > 0 && io_ok(xyzq) && forces_ok &&
-                         c->gtab_valid;
+                         gtab_current(c);
   gse_context_t::FwdKey key;
   key.n = n;
   key.x = xyzq;
@@ -1575,14 +1587,7 @@ gse_status_t gse_virial(gse_context_t* c, double* virial) {
     c->fixed_pending = false;
   }
   const GreenGeom g = green_geom(c, c->sigma2, c->p.box_x, c->p.box_y, c->p.box_z, false);
-  if (!c->d_gtab) CU(cudaMalloc(&c->d_gtab, c->ksize * c->ct));
-  if (!c->gtab_valid) {
-    if (c->fp64)
-      CU(launch_green_table<double>(g, (double*)c->d_gtab, c->stream));
-    else
-      CU(launch_green_table<float>(g, (float*)c->d_gtab, c->stream));
-    c->gtab_valid = true;
-  }
+  TRY(ensure_gtab(c));
   TRY(fft_forward(c, c->d_rho, c->d_rhok));
   const int nb = std::min(sm_count() * 2, kEnergyPartials / 6);
   unsigned* done = reinterpret_cast<unsigned*>(c->d_partials + kEnergyPartials);
