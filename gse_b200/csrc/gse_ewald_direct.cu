@@ -201,11 +201,13 @@ __global__ void __launch_bounds__(kEwdThreads, 2)
               if (hit[u]) q[nq[u] + __popc(m & ((1u << lane) - 1u))] = (unsigned short)j;
               nq[u] += __popc(m);
               if (nq[u] >= 32) {  // uniform in the warp
-                __syncwarp();
-                const int jj = q[lane], rest = q[32 + lane];
-                __syncwarp();
-                q[lane] = (unsigned short)rest;
                 nq[u] -= 32;
+                __syncwarp();
+                const int jj = q[lane], rest = lane < nq[u] ? q[32 + lane] : 0;
+                __syncwarp();
+                // only what is left moves: the next step's lanes write from q[nq] on,
+                // with no barrier between
+                if (lane < nq[u]) q[lane] = (unsigned short)rest;
                 term(u, jj);
               }
             }
