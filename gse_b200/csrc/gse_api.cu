@@ -223,8 +223,9 @@ struct gse_context {
   // the legacy default stream cannot be captured: calls on it are captured on this
   // stream and the graph is launched into theirs
   cudaStream_t cap_stream = nullptr;
-  // classification of the pointers of the captured call, for the replay path
-  bool fwd_host_io = false, fwd_e_host = false;
+  // classification of the pointers of the captured call, for the replay path;
+  // fwd_pinned: those of x, fx, fy, fz that are page-locked host memory
+  bool fwd_host_io = false, fwd_e_host = false, fwd_pinned[4] = {};
   const double* fwd_e_raw = nullptr;
   // optional per-stage device timing (gse_set_timing)
   bool timing = false;
@@ -1171,11 +1172,19 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
   TRY(check_ctx(c));
   // A repeat of the captured call (same count, positions, forces, box and
   // stream) replays its graph: its pointers were checked and classified when
-  // it was captured.  Only a host energy may change address between calls.
+  // it was captured.  Only a host energy may change address between calls.  Host
+  // memory is looked up again: an address that was page-locked may be pageable by now
+  // (unregistered, or freed and given out again), which the graph's copies must not meet.
   const gse_context_t::FwdKey& k = c->fwd_key;
+  auto still_pinned = [&] {
+    const void* p[4] = {xyzq, fx, fy, fz};
+    for (int i = 0; i < 4; i++)
+      if (c->fwd_pinned[i] && !is_pinned_host(p[i])) return false;
+    return true;
+  };
   if (c->fwd_exec && !c->timing && n == k.n && xyzq == k.x && fx == k.fx && fy == k.fy &&
       fz == k.fz && c->stream == k.stream && c->p.box_x == k.box[0] && c->p.box_y == k.box[1] &&
-      c->p.box_z == k.box[2]) {
+      c->p.box_z == k.box[2] && still_pinned()) {
     bool he = c->fwd_e_host;
     if (energy != c->fwd_e_raw) {
       TRY(check_ptr(energy, c->p.device, 1, "energy"));
@@ -1246,14 +1255,7 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
     if (host_e) *energy = c->h_pinned[0];
     return GSE_OK;
   };
-  if (c->fwd_exec && key == c->fwd_key) {
-    CU(cudaGraphLaunch(c->fwd_exec, c->stream));
-    c->fwd_replays++;
-    c->launches += c->fwd_launches;
-    c->rho_valid = c->phi_valid = c->energy_valid = true;
-    return done(host_io);
-  }
-  if (!(key == c->fwd_key)) {
+  if (!(key == c->fwd_key) || c->fwd_exec) {
     // first call with this key: run it directly and remember the key.  A capture costs
     // some ten calls; a program whose buffers change sooner than that is left alone
     // for longer each time.
@@ -1296,6 +1298,8 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
       c->fwd_host_io = host_io;
       c->fwd_e_host = host_e;
       c->fwd_e_raw = energy;
+      const void* io[4] = {xyzq, fx, fy, fz};
+      for (int i = 0; i < 4; i++) c->fwd_pinned[i] = is_pinned_host(io[i]);
       const cudaError_t el = cudaGraphLaunch(c->fwd_exec, c->stream);
       if (el != cudaSuccess) result = fail(GSE_ERR_CUDA, "cudaGraphLaunch: %s", cudaGetErrorString(el));
     } else {
