@@ -318,9 +318,14 @@ gse_status_t use_stream(gse_context_t* c, cudaStream_t st) {
   return GSE_OK;
 }
 
-// Forget the captured forward graph (its buffers or parameters change).
+// Forget the captured forward graph (its buffers or parameters change).  A capture
+// costs some ten calls: a program that loses its graphs sooner than they repay that,
+// by whatever call, is left alone for longer each time.
 void drop_fwd_graph(gse_context_t* c) {
-  if (c->fwd_exec) cudaGraphExecDestroy(c->fwd_exec);
+  if (c->fwd_exec) {
+    c->fwd_need = c->fwd_replays >= 16 ? 1 : std::min(64, 4 * c->fwd_need);
+    cudaGraphExecDestroy(c->fwd_exec);
+  }
   c->fwd_exec = nullptr;
   c->fwd_key = gse_context_t::FwdKey();
 }
@@ -1256,10 +1261,7 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
     return GSE_OK;
   };
   if (!(key == c->fwd_key) || c->fwd_exec) {
-    // first call with this key: run it directly and remember the key.  A capture costs
-    // some ten calls; a program whose buffers change sooner than that is left alone
-    // for longer each time.
-    if (c->fwd_exec) c->fwd_need = c->fwd_replays >= 16 ? 1 : std::min(64, 4 * c->fwd_need);
+    // first call with this key: run it directly and remember the key
     drop_fwd_graph(c);
     TRY(body(&host));
     c->fwd_key = key;
