@@ -184,6 +184,8 @@ struct gse_context {
   volatile int* h_bad = nullptr;
   int* d_badmap = nullptr;
   cufftHandle plan_f = 0, plan_b = 0;
+  cudaStream_t plan_stream = nullptr;  // where the plans run, when plans_moved
+  bool plans_moved = true;
   bool plans = false;
   // c2r plan whose load callback multiplies by the Green's table (the solve
   // of the context's own sigma2 and box; plan_b stays plain for the others)
@@ -308,13 +310,16 @@ gse_status_t check_stencil(const gse_context_t* c, const double box[3], double s
   return GSE_OK;
 }
 
-// All work of the context on `st` from here on.
-gse_status_t use_stream(gse_context_t* c, cudaStream_t st) {
-  if (c->stream == st) return GSE_OK;
-  c->stream = st;
-  CUFFT(cufftSetStream(c->plan_f, st));
-  CUFFT(cufftSetStream(c->plan_b, st));
-  if (c->green_cb) CUFFT(cufftSetStream(c->plan_bg, st));
+// The cuFFT plans on the context's stream.  Called where plans run, so that one which
+// could not be moved runs nowhere else: the call fails, and the next one tries again.
+gse_status_t plans_on_stream(gse_context_t* c) {
+  if (c->plans_moved && c->plan_stream == c->stream) return GSE_OK;
+  c->plans_moved = false;
+  CUFFT(cufftSetStream(c->plan_f, c->stream));
+  CUFFT(cufftSetStream(c->plan_b, c->stream));
+  if (c->green_cb) CUFFT(cufftSetStream(c->plan_bg, c->stream));
+  c->plan_stream = c->stream;
+  c->plans_moved = true;
   return GSE_OK;
 }
 
@@ -504,6 +509,7 @@ double energy_factor(const gse_context_t* c) {
 }
 
 gse_status_t fft_forward(gse_context_t* c, const void* rho, void* rhok) {
+  TRY(plans_on_stream(c));
   if (c->fp64)
     CUFFT(cufftExecD2Z(c->plan_f, (cufftDoubleReal*)rho, (cufftDoubleComplex*)rhok));
   else
@@ -512,6 +518,7 @@ gse_status_t fft_forward(gse_context_t* c, const void* rho, void* rhok) {
 }
 
 gse_status_t fft_backward(gse_context_t* c, void* rhok, void* phi) {
+  TRY(plans_on_stream(c));
   if (c->fp64)
     CUFFT(cufftExecZ2D(c->plan_b, (cufftDoubleComplex*)rhok, (cufftDoubleReal*)phi));
   else
@@ -561,8 +568,7 @@ bool make_green_callback_plan(gse_context_t* c) {
                             c->fp64 ? CUFFT_CB_LD_COMPLEX_DOUBLE : CUFFT_CB_LD_COMPLEX,
                             &c->d_gtab) == CUFFT_SUCCESS &&
       cufftMakePlan3d(pl, c->p.size_z, c->p.size_y, c->p.size_x,
-                      c->fp64 ? CUFFT_Z2D : CUFFT_C2R, &ws) == CUFFT_SUCCESS &&
-      cufftSetStream(pl, c->stream) == CUFFT_SUCCESS;
+                      c->fp64 ? CUFFT_Z2D : CUFFT_C2R, &ws) == CUFFT_SUCCESS;
   if (!ok) {
     cufftDestroy(pl);
     cudaGetLastError();
@@ -643,6 +649,7 @@ gse_status_t do_solve_ctx(gse_context_t* c) {
     if (cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
       c->green_cb = make_green_callback_plan(c);
       c->green_cb_tried = true;
+      if (c->green_cb) c->plans_moved = false;
     }
     cudaGetLastError();
   }
@@ -1026,7 +1033,8 @@ gse_status_t gse_set_stream(gse_context_t* c, void* stream) {
   TRY(check_ctx(c));
   if (c->stream == (cudaStream_t)stream) return GSE_OK;
   drop_fwd_graph(c);
-  return use_stream(c, (cudaStream_t)stream);
+  c->stream = (cudaStream_t)stream;
+  return plans_on_stream(c);
 }
 
 gse_status_t gse_set_box(gse_context_t* c, double bx, double by, double bz) {
@@ -1276,21 +1284,24 @@ gse_status_t gse_forward(gse_context_t* c, int n, const void* xyzq, double* ener
   // the next identical call: capture, instantiate, launch
   const long long l0 = c->launches;
   const cudaStream_t user = c->stream;
-  if (!user) {
-    if (!c->cap_stream)
-      CU(cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
-    TRY(use_stream(c, c->cap_stream));
-  }
   cudaGraph_t g = nullptr;
   gse_status_t st = GSE_OK;
-  cudaError_t ec = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
-  if (ec == cudaSuccess) {
-    st = body(&host);
-    ec = cudaStreamEndCapture(c->stream, &g);
-  } else if (user) {
-    return fail(GSE_ERR_CUDA, "cudaStreamBeginCapture: %s", cudaGetErrorString(ec));
+  cudaError_t ec = cudaSuccess;
+  if (!user) {
+    if (!c->cap_stream) ec = cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking);
+    if (ec == cudaSuccess) c->stream = c->cap_stream;
   }
-  TRY(use_stream(c, user));
+  if (ec == cudaSuccess) st = plans_on_stream(c);
+  if (ec == cudaSuccess && st == GSE_OK) {
+    ec = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+    if (ec == cudaSuccess) {
+      st = body(&host);
+      ec = cudaStreamEndCapture(c->stream, &g);
+    } else if (user) {
+      return fail(GSE_ERR_CUDA, "cudaStreamBeginCapture: %s", cudaGetErrorString(ec));
+    }
+  }
+  c->stream = user;
   c->fwd_replays = 0;
   gse_status_t result = st;
   if (st == GSE_OK && ec == cudaSuccess) {
