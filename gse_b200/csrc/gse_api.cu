@@ -592,6 +592,7 @@ gse_status_t own_solve(gse_context_t* c, bool fixed, float* rho_out, float* phi,
                                  fixed ? nullptr : (const float*)c->d_rho,
                                  std::exp2(-(double)kFlushBits), rho_out, (float2*)c->d_rhok,
                                  c->d_fft_tw, c->bl.flags, pdl, c->fft_stall_test, c->stream));
+    c->fixed_pending = false;  // a deferred density is in the float grid now
   }
   {
     StageTimer tm(c, GSE_STAGE_GREEN);
@@ -640,7 +641,6 @@ gse_status_t do_solve_ctx(gse_context_t* c) {
     // launches, unless stage timing puts events between them
     TRY(own_solve(c, fx, fx ? (float*)c->d_rho : nullptr, (float*)c->d_phi, c->d_scalars,
                   fx && !c->timing));
-    c->fixed_pending = false;
     return GSE_OK;
   }
   if (!c->green_cb_tried && c->size >= kGreenCallbackMinPoints) {
@@ -1368,6 +1368,7 @@ gse_status_t gse_set_grid(gse_context_t* c, int which, const void* in) {
   if (which == GSE_GRID_RHO) {
     c->rho_valid = true;
     c->phi_valid = false;
+    c->fixed_pending = false;
   } else {
     c->phi_valid = true;
   }
