@@ -1924,10 +1924,23 @@ gse_status_t gse_ewald_recip(int device, void* stream, double sigma, int kcut, d
   }
   const bool xdev = is_device_ptr(xyzq);
   const bool fdev = want_f && is_device_ptr(fx) && is_device_ptr(fy) && is_device_ptr(fz);
-  // one allocation: the sums' scratch, then staged atoms and forces
-  const EwPlan plan = ewald_plan(n, kcut, (int)rows.size(), want_f);
-  const size_t off_x = plan.bytes, off_f = off_x + (xdev ? 0 : sizeof(double4) * (size_t)n);
-  CUE(scratch.take(device, off_f + (want_f && !fdev ? sizeof(double) * 3 * (size_t)n : 0)));
+  // one allocation: the sums' scratch, then staged atoms and forces.  Where the device is
+  // short of memory the sums go in smaller pieces, down to 2 MB.
+  EwPlan plan;
+  size_t off_x = 0, off_f = 0;
+  for (size_t budget = kEwBudget;; budget /= 4) {
+    plan = ewald_plan(n, rows, kcut, want_f, budget);
+    off_x = plan.bytes;
+    off_f = off_x + (xdev ? 0 : sizeof(double4) * (size_t)n);
+    const cudaError_t e =
+        scratch.take(device, off_f + (want_f && !fdev ? sizeof(double) * 3 * (size_t)n : 0));
+    if (e == cudaErrorMemoryAllocation && budget > (2u << 20)) {
+      cudaGetLastError();
+      continue;
+    }
+    CUE(e);
+    break;
+  }
   char* buf = scratch.buf;
   const double4* xin = (const double4*)xyzq;
   if (!xdev) {

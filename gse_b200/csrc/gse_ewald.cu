@@ -372,15 +372,17 @@ __global__ void __launch_bounds__(kEwThreads)
   }
 }
 
-// Forces of the slab from the row splits, in split order.
+// Forces of the slab from the row splits, in split order (add: to the former blocks').
 __global__ void k_ewald_force_sum(const double* __restrict__ fpart, int nsplit, int pitch, int na,
-                                  EwGeom g, double* __restrict__ fx, double* __restrict__ fy,
-                                  double* __restrict__ fz) {
+                                  EwGeom g, bool add, double* __restrict__ fx,
+                                  double* __restrict__ fy, double* __restrict__ fz) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x, d = blockIdx.y;
   if (a >= na) return;
   double s = 0.0;
   for (int w = 0; w < nsplit; w++) s += fpart[((long long)w * 3 + d) * pitch + a];
-  (d == 0 ? fx : d == 1 ? fy : fz)[a] = 4.0 * 2.0 * kPi * g.inv_box[d] * s;
+  s *= 4.0 * 2.0 * kPi * g.inv_box[d];
+  double* f = (d == 0 ? fx : d == 1 ? fy : fz) + a;
+  *f = add ? *f + s : s;
 }
 
 std::vector<EwRow> ewald_rows(int kcut) {
@@ -406,41 +408,73 @@ std::vector<EwRow> ewald_rows(int kcut) {
 // beyond (the largest kcut's table fits no more).
 static bool ew_wide(int wpitch) { return wpitch <= 128; }
 
-EwPlan ewald_plan(int n, int kcut, int nrows, bool forces) {
+EwPlan ewald_plan(int n, const std::vector<EwRow>& rows, int kcut, bool forces, size_t budget) {
   EwPlan p;
   p.kmax = kcut;
-  p.nrows = nrows;
-  p.ncols = (2 * (kcut + 1) + 7) / 8 * 8;
-  p.wpitch = (2 * (kcut + 1) + kEwFK - 1) / kEwFK * kEwFK;
-  // atoms per slab: the phase tables (48 bytes per atom and k) within 256 MB
-  const long long most = (256ll << 20) / (48ll * (kcut + 1));
-  p.slab = (int)std::min<long long>(n, std::max<long long>(4096, most / 64 * 64));
+  p.nrows = (int)rows.size();
+  // atoms per slab: the phase tables (48 bytes per atom and k) within half the budget
+  const long long half = (long long)(budget / 2), most = half / (48ll * (kcut + 1));
+  p.slab = (int)std::min<long long>(n, std::max<long long>(64, most / 64 * 64));
   p.pitch = (p.slab + 63) / 64 * 64;
   const int sms = sm_count();
-  // atom splits of the structure kernel: four blocks per SM slot pair
-  const int blocks = (nrows + kEwRows - 1) / kEwRows * ((p.ncols + kEwCols - 1) / kEwCols);
-  int ks = std::max(1, std::min(16, 4 * sms / blocks));
-  ks = std::min(ks, std::max(1, p.pitch / (4 * kEwChunk)));
-  p.per_split = ((p.pitch + ks - 1) / ks + kEwChunk - 1) / kEwChunk * kEwChunk;
-  p.nsplit = (p.pitch + p.per_split - 1) / p.per_split;
-  // row splits of the force kernel: at least twelve blocks per SM
-  const int mt = ew_wide(p.wpitch) ? 64 : 32;
-  const int fb = (p.pitch + mt - 1) / mt;
-  int rs = std::max(1, std::min(32, 12 * sms / fb));
-  p.per_fsplit = ((nrows + rs - 1) / rs + kEwFRows - 1) / kEwFRows * kEwFRows;
-  p.nfsplit = (nrows + p.per_fsplit - 1) / p.per_fsplit;
+  auto block = [&](int row0, int nrows) {
+    EwBlock b;
+    b.row0 = row0;
+    b.nrows = nrows;
+    const int k2 = 2 * (rows[row0].kxm + 1);  // of its longest row
+    b.ncols = (k2 + 7) / 8 * 8;
+    b.wpitch = (k2 + kEwFK - 1) / kEwFK * kEwFK;
+    // atom splits of the structure kernel: four blocks per SM slot pair, the splits'
+    // sums within a quarter of the budget
+    const int blocks = (nrows + kEwRows - 1) / kEwRows * ((b.ncols + kEwCols - 1) / kEwCols);
+    int ks = std::max(1, std::min(16, 4 * sms / blocks));
+    ks = std::min(ks, std::max(1, p.pitch / (4 * kEwChunk)));
+    ks = (int)std::min<long long>(ks, std::max(1ll, half / 2 / (16ll * nrows * b.ncols)));
+    b.per_split = ((p.pitch + ks - 1) / ks + kEwChunk - 1) / kEwChunk * kEwChunk;
+    b.nsplit = (p.pitch + b.per_split - 1) / b.per_split;
+    // row splits of the force kernel: at least twelve blocks per SM
+    const int mt = ew_wide(b.wpitch) ? 64 : 32;
+    const int fb = (p.pitch + mt - 1) / mt;
+    const int rs = std::max(1, std::min(32, 12 * sms / fb));
+    b.per_fsplit = ((nrows + rs - 1) / rs + kEwFRows - 1) / kEwFRows * kEwFRows;
+    b.nfsplit = (nrows + b.per_fsplit - 1) / b.per_fsplit;
+    return b;
+  };
+  auto part_bytes = [](const EwBlock& b) {
+    return sizeof(double) * 2 * (size_t)b.nsplit * b.nrows * b.ncols;
+  };
+  auto w_bytes = [&](const EwBlock& b) {
+    return forces ? sizeof(double4) * (size_t)b.nrows * b.wpitch : 0;
+  };
+  // rows per block: all of them unless their sums (32 bytes per kx and sign for the
+  // forces, 16 per split for S) exceed half the budget, from about kcut 120 on; 2.4 GB
+  // at kcut 255 in one block
+  int per = p.nrows;
+  while (per > kEwRows) {
+    const EwBlock b = block(0, per);
+    if (part_bytes(b) + w_bytes(b) <= (size_t)half) break;
+    per = std::max(kEwRows, (per / 2 + kEwRows - 1) / kEwRows * kEwRows);
+  }
+  size_t part = 0, w = 0, f = 0;
+  for (int r = 0; r < p.nrows; r += per) {
+    const EwBlock b = block(r, std::min(per, p.nrows - r));
+    part = std::max(part, part_bytes(b));
+    w = std::max(w, w_bytes(b));
+    if (forces) f = std::max(f, sizeof(double) * 3 * (size_t)b.nfsplit * p.pitch);
+    p.blocks.push_back(b);
+  }
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t o = off;
     off = (off + bytes + 255) / 256 * 256;
     return o;
   };
-  p.off_rows = take(sizeof(EwRow) * nrows);
-  p.off_energy = take(sizeof(double) * nrows);
+  p.off_rows = take(sizeof(EwRow) * p.nrows);
+  p.off_energy = take(sizeof(double) * p.nrows);
   p.off_T = take(sizeof(double2) * 3 * (size_t)(kcut + 1) * p.pitch);
-  p.off_part = take(sizeof(double) * 2 * (size_t)p.nsplit * nrows * p.ncols);
-  p.off_W = forces ? take(sizeof(double4) * (size_t)nrows * p.wpitch) : 0;
-  p.off_f = forces ? take(sizeof(double) * 3 * (size_t)p.nfsplit * p.pitch) : 0;
+  p.off_part = take(part);
+  p.off_W = take(w);
+  p.off_f = take(f);
   p.bytes = off;
   return p;
 }
@@ -448,42 +482,48 @@ EwPlan ewald_plan(int n, int kcut, int nrows, bool forces) {
 cudaError_t launch_ewald(const double4* xyzq, int n, const std::vector<EwRow>& rows,
                          const EwGeom& g, const EwPlan& p, char* buf, double* fx, double* fy,
                          double* fz, cudaStream_t st) {
-  const int nrows = p.nrows;
   EwRow* rows_d = (EwRow*)(buf + p.off_rows);
   double2* T = (double2*)(buf + p.off_T);
   double* part = (double*)(buf + p.off_part);
   double4* Wt = fx ? (double4*)(buf + p.off_W) : nullptr;
   double* fpart = (double*)(buf + p.off_f);
-  cudaError_t e = cudaMemcpyAsync(rows_d, rows.data(), sizeof(EwRow) * nrows,
+  cudaError_t e = cudaMemcpyAsync(rows_d, rows.data(), sizeof(EwRow) * p.nrows,
                                   cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
+  // the tables of one slab stay for everything that follows when there is one only
+  bool have = false;
   auto tables = [&](int a0) {
     const int na = std::min(p.slab, n - a0);
-    k_ewald_tables<<<dim3(p.pitch / 64, 3), 256, 0, st>>>(xyzq + a0, na, p.pitch, p.kmax, g, T);
+    if (!have)
+      k_ewald_tables<<<dim3(p.pitch / 64, 3), 256, 0, st>>>(xyzq + a0, na, p.pitch, p.kmax, g, T);
+    have = p.slab >= n;
     return na;
   };
-  const dim3 sg((nrows + kEwRows - 1) / kEwRows, (p.ncols + kEwCols - 1) / kEwCols, p.nsplit);
-  for (int a0 = 0; a0 < n; a0 += p.slab) {
-    tables(a0);
-    k_ewald_structure<<<sg, kEwThreads, 0, st>>>(T, p.pitch, p.kmax, rows_d, nrows, p.per_split,
-                                                 p.ncols, a0 > 0, part);
-  }
-  k_ewald_finish<<<(nrows + 7) / 8, 256, 0, st>>>(part, p.nsplit, p.ncols, rows_d, nrows, g,
-                                                  p.wpitch, Wt, (double*)(buf + p.off_energy));
-  if (fx) {
-    const bool wide = ew_wide(p.wpitch);
+  for (const EwBlock& b : p.blocks) {
+    const EwRow* r = rows_d + b.row0;
+    const dim3 sg((b.nrows + kEwRows - 1) / kEwRows, (b.ncols + kEwCols - 1) / kEwCols, b.nsplit);
+    for (int a0 = 0; a0 < n; a0 += p.slab) {
+      tables(a0);
+      k_ewald_structure<<<sg, kEwThreads, 0, st>>>(T, p.pitch, p.kmax, r, b.nrows, b.per_split,
+                                                   b.ncols, a0 > 0, part);
+    }
+    k_ewald_finish<<<(b.nrows + 7) / 8, 256, 0, st>>>(part, b.nsplit, b.ncols, r, b.nrows, g,
+                                                      b.wpitch, Wt,
+                                                      (double*)(buf + p.off_energy) + b.row0);
+    if (!fx) continue;
+    const bool wide = ew_wide(b.wpitch);
     const int mt = wide ? 64 : 32;
     const size_t smem =
-        sizeof(double) * ((size_t)p.wpitch * (mt + 4) + 2 * kEwFK * kEwFPitch);
+        sizeof(double) * ((size_t)b.wpitch * (mt + 4) + 2 * kEwFK * kEwFPitch);
     auto kernel = wide ? k_ewald_force<2, 4> : k_ewald_force<2, 2>;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     for (int a0 = 0; a0 < n; a0 += p.slab) {
-      const int na = p.slab < n ? tables(a0) : n;
-      kernel<<<dim3((p.pitch + mt - 1) / mt, p.nfsplit), kEwThreads, smem, st>>>(
-          T, p.pitch, p.kmax, rows_d, nrows, p.per_fsplit, p.wpitch, Wt, fpart);
+      const int na = tables(a0);
+      kernel<<<dim3((p.pitch + mt - 1) / mt, b.nfsplit), kEwThreads, smem, st>>>(
+          T, p.pitch, p.kmax, r, b.nrows, b.per_fsplit, b.wpitch, Wt, fpart);
       k_ewald_force_sum<<<dim3((na + 255) / 256, 3), 256, 0, st>>>(
-          fpart, p.nfsplit, p.pitch, na, g, fx + a0, fy + a0, fz + a0);
+          fpart, b.nfsplit, p.pitch, na, g, b.row0 > 0, fx + a0, fy + a0, fz + a0);
     }
   }
   return cudaGetLastError();

@@ -19,20 +19,31 @@ struct EwRow {
   int ky, kz, kx0, kxm;
 };
 
+// A run of rows whose sums are in the scratch at one time.
+struct EwBlock {
+  int row0, nrows;
+  int ncols;   // columns of S: c, s of every kx, whole 8-column strips
+  int wpitch;  // the same for the force kernel, whole chunks
+  int per_split, nsplit;    // atoms per split of the structure sum
+  int per_fsplit, nfsplit;  // rows per split of the force sum
+};
+
 // Sizes and scratch layout of one call (one allocation of `bytes`).
 struct EwPlan {
   int kmax, nrows;
-  int ncols;       // columns of S: c, s of every kx, whole 8-column strips
-  int wpitch;      // the same for the force kernel, whole chunks
-  int slab, pitch; // atoms per pass, and rounded up to 64
-  int per_split, nsplit;    // atoms per split of the structure sum
-  int per_fsplit, nfsplit;  // rows per split of the force sum
+  int slab, pitch;  // atoms per pass, and rounded up to 64
+  std::vector<EwBlock> blocks;
   size_t off_rows, off_energy, off_T, off_part, off_W, off_f, bytes;
 };
 
 // Rows of the half sphere |k| <= kcut, longest first.
 std::vector<EwRow> ewald_rows(int kcut);
-EwPlan ewald_plan(int n, int kcut, int nrows, bool forces);
+// `budget`: bytes of scratch to plan for, half of it for the phase tables (more atoms
+// go in slabs) and half for the rows' sums (more rows go in blocks); at least 64 atoms
+// and 32 rows at a time.  The rows themselves, 24 bytes each, and the forces' partial
+// sums, a few MB, come on top.
+constexpr size_t kEwBudget = 512ull << 20;
+EwPlan ewald_plan(int n, const std::vector<EwRow>& rows, int kcut, bool forces, size_t budget);
 // `buf`: p.bytes of device memory; the rows' energies are left at p.off_energy.
 cudaError_t launch_ewald(const double4* xyzq, int n, const std::vector<EwRow>& rows,
                          const EwGeom& g, const EwPlan& p, char* buf, double* fx, double* fy,

@@ -257,7 +257,8 @@ gse_status_t gse_adjoint(gse_context_t* ctx, int n, const void* xyzq, double dLd
 /* ---- Ewald reference sum --------------------------------------------------- */
 /* The two calls below take their scratch from a memory pool of the library's own,
  * one per device, which keeps up to 256 MB between calls.  They synchronise the
- * stream; calls of several threads and streams may overlap. */
+ * stream; calls of several threads and streams may overlap.  The reciprocal sum takes
+ * up to about 0.5 GB, and where the device has less it works in smaller pieces. */
 
 /* CpuEwaldRecip::calcForceEnergy (CpuEwaldRecip.cpp:87-147) on the GPU in FP64:
  * E = sum over integer k != 0 with |k|^2 <= kcut^2 of
