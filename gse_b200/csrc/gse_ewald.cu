@@ -406,7 +406,12 @@ std::vector<EwRow> ewald_rows(int kcut) {
 
 // Force blocks of 64 atoms while their x table leaves room for two blocks per SM, 32
 // beyond (the largest kcut's table fits no more).
-static bool ew_wide(int wpitch) { return wpitch <= 128; }
+constexpr int kEwWide = 128;  // of wpitch
+static bool ew_wide(int wpitch) { return wpitch <= kEwWide; }
+
+static size_t ew_force_smem(int wpitch, int mt) {
+  return sizeof(double) * ((size_t)wpitch * (mt + 4) + 2 * kEwFK * kEwFPitch);
+}
 
 EwPlan ewald_plan(int n, const std::vector<EwRow>& rows, int kcut, bool forces, size_t budget) {
   EwPlan p;
@@ -513,10 +518,11 @@ cudaError_t launch_ewald(const double4* xyzq, int n, const std::vector<EwRow>& r
     if (!fx) continue;
     const bool wide = ew_wide(b.wpitch);
     const int mt = wide ? 64 : 32;
-    const size_t smem =
-        sizeof(double) * ((size_t)b.wpitch * (mt + 4) + 2 * kEwFK * kEwFPitch);
+    const size_t smem = ew_force_smem(b.wpitch, mt);
     auto kernel = wide ? k_ewald_force<2, 4> : k_ewald_force<2, 2>;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit is the kernel's, not this call's: calls of other threads share it
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)ew_force_smem(wide ? kEwWide : 2 * 256, mt));
     if (e != cudaSuccess) return e;
     for (int a0 = 0; a0 < n; a0 += p.slab) {
       const int na = tables(a0);
