@@ -2028,11 +2028,15 @@ gse_status_t gse_ewald_direct(int device, void* stream, double sigma, double rcu
   const EwdGeom g = ewald_direct_geom(sigma, rcut, box, ccelec);
   const int ntiles = (g.ncell + 4095) / 4096;
   // one allocation: ints, then doubles (8-byte aligned), then atoms
-  const size_t n_int = 2 * (size_t)n + (size_t)g.ncell * 3 + 1 + ntiles + n + 1 + ex_idx.size() +
-                       (ex_start.empty() ? 0 : n + 1);
+  const size_t n_cells = std::min(n, g.ncell);
+  // (the exclusions on boundaries of 128 bytes: their copies from pageable memory took
+  // 30 us longer at odd ones)
+  const size_t off_ex =
+      (3 * (size_t)n + (size_t)g.ncell * 3 + 1 + ntiles + n_cells + 2 + 31) / 32 * 32;
+  const size_t off_es = off_ex + (ex_idx.size() + 31) / 32 * 32;
+  const size_t n_int = off_es + (ex_start.empty() ? 0 : n + 1);
   const size_t off_d = (n_int * sizeof(int) + 31) / 32 * 32;
-  const size_t n_part = (size_t)g.ncell * ewald_direct_split(n, g);
-  const size_t n_dbl = n_part + 1 + (want_f ? 3 * (size_t)n : 0);
+  const size_t n_dbl = n + 1 + (want_f ? 3 * (size_t)n : 0);
   const size_t off_x = (off_d + n_dbl * sizeof(double) + 31) / 32 * 32;
   const bool xdev = is_device_ptr(xyzq);
   const size_t bytes = off_x + (size_t)n * sizeof(double4) * (xdev ? 1 : 2);
@@ -2070,14 +2074,14 @@ gse_status_t gse_ewald_direct(int device, void* stream, double sigma, double rcu
   ip += g.ncell;
   w.perm = ip;
   ip += n;
+  w.cells = ip;
+  ip += n_cells;
   w.done = (unsigned*)ip;
-  ip += 1;
-  int* d_ex_idx = ip;
-  ip += ex_idx.size();
-  int* d_ex_start = ex_start.empty() ? nullptr : ip;
+  int* d_ex_idx = (int*)buf + off_ex;
+  int* d_ex_start = ex_start.empty() ? nullptr : (int*)buf + off_es;
   double* dp = (double*)(buf + off_d);
   w.partials = dp;
-  double* d_energy = dp + n_part;
+  double* d_energy = dp + n;
   double* f[3] = {fx, fy, fz};
   const bool fdev = want_f && is_device_ptr(fx) && is_device_ptr(fy) && is_device_ptr(fz);
   if (want_f && !fdev)

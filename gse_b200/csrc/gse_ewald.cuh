@@ -71,15 +71,14 @@ struct EwdScratch {
   int* tmp;         // [n]
   double4* sorted;  // [n] atoms in cell order
   int* perm;        // [n] original index of each sorted atom
-  double* partials; // [ncell * split] energy per block
-  unsigned* done;   // counter of finished blocks
+  int* cells;       // [min(n, ncell)] cells that hold atoms
+  double* partials; // [n] energies of the blocks
+  unsigned* done;   // [2] counters of finished blocks and of such cells
 };
 
 EwdGeom ewald_direct_geom(double sigma, double rcut, const double box[3], double ccelec);
-// Blocks per cell of the pair kernel.
-int ewald_direct_split(int n, const EwdGeom& g);
 // ex_start[n + 1] / ex_idx: the excluded partners of every atom (both
-// directions), or both NULL.  energy_out: one device double.
+// directions), or both NULL.  energy_out: one device double.  n > 0.
 cudaError_t launch_ewald_direct(const double4* xyzq, int n, const EwdGeom& g, EwdScratch w,
                                 const int* ex_start, const int* ex_idx, double* fx, double* fy,
                                 double* fz, double* energy_out, cudaStream_t st);

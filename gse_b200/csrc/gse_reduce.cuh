@@ -7,9 +7,9 @@
 namespace gse {
 
 // ---------------------------------------------------------------------------
-// Block reduction of a double into partials[blockIdx.x] (fixed order).
+// Block reduction of a double into *out, and into partials[blockIdx.x] (fixed order).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void block_sum_to(double v, double* partials) {
+__device__ __forceinline__ void block_sum_at(double v, double* out) {
   __shared__ double red[32];
   v = warp_sum(v);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -18,8 +18,11 @@ __device__ __forceinline__ void block_sum_to(double v, double* partials) {
   if (w == 0) {
     double s = (lane < (int)(blockDim.x >> 5)) ? red[lane] : 0.0;
     s = warp_sum(s);
-    if (lane == 0) partials[blockIdx.x] = s;
+    if (lane == 0) *out = s;
   }
+}
+__device__ __forceinline__ void block_sum_to(double v, double* partials) {
+  block_sum_at(v, partials + blockIdx.x);
 }
 
 // This thread's share (threadIdx.x, threadIdx.x + blockDim.x, ...) of the sum of
@@ -38,10 +41,10 @@ __device__ __forceinline__ double partials_share(const double* p, unsigned n) {
 }
 
 // After block_sum_to: the block that finishes last (a counter at `done`, zero
-// between launches) adds the partials in index order -- the result does not
+// between launches) adds the n partials in index order -- the result does not
 // depend on which block ran when -- and writes factor * sum to out[0].
-__device__ __forceinline__ void last_block_sum_counter(double* partials, unsigned* done,
-                                                       double factor, double* out) {
+__device__ __forceinline__ void last_block_sum_n(double* partials, unsigned n, unsigned* done,
+                                                 double factor, double* out) {
   __shared__ bool last;
   if (threadIdx.x == 0) {
     __threadfence();
@@ -51,7 +54,7 @@ __device__ __forceinline__ void last_block_sum_counter(double* partials, unsigne
   if (!last) return;  // uniform in the block
   __threadfence();
   __shared__ double red[32];
-  const double t = warp_sum(partials_share(partials, gridDim.x));
+  const double t = warp_sum(partials_share(partials, n));
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) red[w] = t;
   __syncthreads();
@@ -63,6 +66,11 @@ __device__ __forceinline__ void last_block_sum_counter(double* partials, unsigne
       *done = 0u;
     }
   }
+}
+// One partial per block.
+__device__ __forceinline__ void last_block_sum_counter(double* partials, unsigned* done,
+                                                       double factor, double* out) {
+  last_block_sum_n(partials, gridDim.x, done, factor, out);
 }
 
 }  // namespace gse
