@@ -307,7 +307,7 @@ cudaError_t launch_ewald_direct(const double4* xyzq, int n, const EwdGeom& g, Ew
   if (e != cudaSuccess) return e;
   // no more cells than atoms hold any: a block per cell of a wide, empty box (1.4 million
   // for 1000 atoms in 100 A at a cut-off of 0.9) took 7.2 ms of launches, 3.8 with the
-  // former kernel's smaller blocks; now 0.26
+  // former kernel's smaller blocks; now 0.13
   const int split = ewald_direct_split(n, g);
   k_ewd_pairs<<<std::min(n, g.ncell) * split, kEwdThreads, smem, st>>>(
       w.sorted, w.perm, w.start, w.cells, w.done + 1, n, g, split, ex_start, ex_idx, fx, fy, fz,
