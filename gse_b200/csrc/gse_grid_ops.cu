@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-template <typename CT>
+template <typename CT, int K>
 __global__ void __launch_bounds__(256)
     k_efield(const CT* __restrict__ phi, CT* __restrict__ ex, CT* __restrict__ ey,
              CT* __restrict__ ez, int mx, int my, int mz, CT ihx, CT ihy, CT ihz) {
@@ -350,11 +350,11 @@ __global__ void __launch_bounds__(256)
   const int y = (int)(r % my), z = (int)(r / my);
   const long long ry = (long long)(y + 1 == my ? 0 : y + 1) * mx + (long long)z * plane;
   const long long rz = (long long)y * mx + (long long)(z + 1 == mz ? 0 : z + 1) * plane;
-  // five x positions per lane and step, their loads issued together
-  for (int xb = 0; xb < mx; xb += 160) {
-    CT c[5], px[5], py[5], pz[5];
+  // K x positions per lane and step, their loads issued together
+  for (int xb = 0; xb < mx; xb += 32 * K) {
+    CT c[K], px[K], py[K], pz[K];
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
+    for (int k = 0; k < K; k++) {
       const int x = xb + threadIdx.x + 32 * k;
       if (x < mx) {
         c[k] = phi[r * mx + x];
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(256)
       }
     }
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
+    for (int k = 0; k < K; k++) {
       const int x = xb + threadIdx.x + 32 * k;
       if (x < mx) {
         const long long p = r * mx + x;
@@ -546,8 +546,14 @@ cudaError_t launch_efield(const CT* phi, CT* ex, CT* ey, CT* ez, const int M[3],
                           const CT inv_h[3], cudaStream_t st) {
   const long long groups = ((long long)M[1] * M[2] + 7) / 8;
   if (groups > 0x7fffffffLL) return cudaErrorInvalidValue;
-  k_efield<CT><<<(unsigned)groups, dim3(32, 8), 0, st>>>(phi, ex, ey, ez, M[0], M[1], M[2],
-                                                          inv_h[0], inv_h[1], inv_h[2]);
+  // Four positions per lane, or five where the row then takes a step less and, in FP64,
+  // nearly fills it.  Four / five in us: FP32 rows of 144 11.4 / 10.8, of 256 49.6 / 51.2;
+  // FP64 rows of 130 15.0 / 16.3, 144 18.4 / 18.9, 160 25.3 / 23.8, 192 38.4 / 39.8.
+  const int s5 = (M[0] + 159) / 160;
+  const bool five = s5 < (M[0] + 127) / 128 && (sizeof(CT) == 4 || 16 * M[0] >= 15 * 160 * s5);
+  auto kernel = five ? k_efield<CT, 5> : k_efield<CT, 4>;
+  kernel<<<(unsigned)groups, dim3(32, 8), 0, st>>>(phi, ex, ey, ez, M[0], M[1], M[2], inv_h[0],
+                                                   inv_h[1], inv_h[2]);
   return cudaGetLastError();
 }
 
