@@ -282,6 +282,14 @@ __global__ void __launch_bounds__(32 * kAdjWarps)
 constexpr int kFusedRevThreads = 512;   // the fused reverse kernel's block
 constexpr int kAdjScatterThreads = 512;  // >= kSB * kSB; 64 registers at two blocks per SM
 
+// Blocks per SM that the source and the gather are built for: two, but one at width 15,
+// whose blocks (126 KB in the source, 141 KB in the gather) leave no room for a
+// second.  Bounded for two all the same, width 15 had 64 and 128 registers instead of 80
+// to 109 and 175 to 200: 128 systems, 407,193 charges, source 0.909 -> 0.741 ms, gather
+// 1.887 -> 1.530; one system of 164,637 charges on 144^3 0.307 -> 0.288 and 0.743 -> 0.600.
+// One block at the other widths: source 0.767 -> 0.853 ms at 13, 0.734 -> 0.779 at 11.
+constexpr int adj_blocks(int W) { return W < 15 ? 2 : 1; }
+
 // Per-warp slots for the y tables of the reverse-pass scatter, one array for
 // every stencil width a kernel instantiates (a static array in the templated
 // function would be one per width, too much static shared memory for the
@@ -696,7 +704,7 @@ __device__ __forceinline__ void adj_gather_brick(
 }
 
 template <int W>
-__global__ void __launch_bounds__(kAdjScatterThreads, 2)
+__global__ void __launch_bounds__(kAdjScatterThreads, adj_blocks(W))
     k_adj_scatter(const float4* __restrict__ sorted, const float4* __restrict__ gs,
                   const int* __restrict__ start, BinLayout b, Stencil<float> s, float cA,
                   int nparts, long long* __restrict__ grid64) {
@@ -707,7 +715,7 @@ __global__ void __launch_bounds__(kAdjScatterThreads, 2)
 }
 
 template <int W>
-__global__ void __launch_bounds__(kAdjThreads, 2)
+__global__ void __launch_bounds__(kAdjThreads, adj_blocks(W))
     k_adj_gather_tiled(const float4* __restrict__ sorted, const int* __restrict__ perm,
                        const int* __restrict__ start, BinLayout b, Stencil<float> sp,
                        Stencil<float> sg, double c, double gE_ch3, const float* __restrict__ psi,
@@ -721,7 +729,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2)
 }
 
 template <int W>
-__global__ void __launch_bounds__(kAdjScatterThreads, 2)
+__global__ void __launch_bounds__(kAdjScatterThreads, adj_blocks(W))
     k_batch_adj_scatter(const float4* __restrict__ sorted, const float4* __restrict__ gs,
                         const int* __restrict__ start, const BatchSys* __restrict__ sys,
                         const BatchItem* __restrict__ items, int nitems, double c,
@@ -738,7 +746,7 @@ __global__ void __launch_bounds__(kAdjScatterThreads, 2)
 }
 
 template <int W>
-__global__ void __launch_bounds__(kAdjThreads, 2)
+__global__ void __launch_bounds__(kAdjThreads, adj_blocks(W))
     k_batch_adj_gather_tiled(const float4* __restrict__ sorted, const int* __restrict__ perm,
                              const int* __restrict__ start, const BatchSys* __restrict__ sys,
                              const BatchItem* __restrict__ items, int nitems, double c,
