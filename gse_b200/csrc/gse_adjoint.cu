@@ -468,14 +468,14 @@ struct AdjGatherGeom {
   static constexpr int TP = TX | 1;
   static constexpr int ZP = ((TY * TP + 31) / 32) * 32 + ((W * TP) % 32);
   static constexpr int NW = NT / 32;
-  static constexpr int APW = 32 / kAdjLanes;  // atoms per warp at a time
   static constexpr size_t bytes =
-      sizeof(float) * (2 * TZ * ZP + NW * APW * 9 * kWPad) + sizeof(int) * NW * APW * W * W;
+      sizeof(float) * (2 * TZ * ZP + NW * 9 * kWPad) + sizeof(int) * NW * W * W;
 };
 
 // Reverse-pass gather of the atoms of one kAX x kAY x kAZ brick: Psi = psi +
-// gE c h^3 phi and phi of the brick plus halo in shared memory; kAdjLanes
-// lanes per atom: the cube rows of Psi (moments e, e u_x) and the sphere rows
+// gE c h^3 phi and phi of the brick plus halo in shared memory; a whole warp
+// per atom (two atoms would need more shared memory than two blocks per SM leave for
+// their tables): the cube rows of Psi (moments e, e u_x) and the sphere rows
 // of phi (moments e, e u_x, e u_x^2), combined into dL/dq and dL/dx.
 template <int W, int NT = kAdjThreads>
 __device__ __forceinline__ void adj_gather_brick(
@@ -488,18 +488,16 @@ __device__ __forceinline__ void adj_gather_brick(
     unsigned char* smem) {
   typedef AdjGatherGeom<W, NT> AG;
   constexpr int n = AG::n, TX = AG::TX, TY = AG::TY, TZ = AG::TZ, TP = AG::TP, ZP = AG::ZP;
-  constexpr int NW = AG::NW, APW = AG::APW, GL = kAdjLanes;
+  constexpr int NW = AG::NW;
   constexpr int NR = kAY * kAZ;
-  constexpr int NG = (W * W + GL - 1) / GL;
+  constexpr int NG = (W * W + 31) / 32;
   float* tpsi = (float*)smem;                        // [TZ][ZP]
   float* tphi = tpsi + TZ * ZP;                      // [TZ][ZP]
-  float* tabs = tphi + TZ * ZP;                      // [NW][APW][axis][u, u^2, e][kWPad]
-  int* rowl = (int*)(tabs + NW * APW * 9 * kWPad);   // [NW][APW][W*W]
-  static_assert(GL == 32, "a warp per atom");
+  float* tabs = tphi + TZ * ZP;                      // [NW][axis][u, u^2, e][kWPad]
+  int* rowl = (int*)(tabs + NW * 9 * kWPad);         // [NW][W*W]
   __shared__ int rng_a[NR], rng_p[NR + 1];
   __shared__ int alist[kGatherList];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int grp = lane / GL, gl = lane % GL;
   const int x0 = bxi * kAX, y0 = byi * kAY, z0 = bzi * kAZ;
   const int ex = min(kAX, b.M[0] - x0), ey = min(kAY, b.M[1] - y0), ez = min(kAZ, b.M[2] - z0);
   int cnt = 0;
@@ -529,16 +527,15 @@ __device__ __forceinline__ void adj_gather_brick(
   }
   __syncthreads();
 
-  float* tb = tabs + (warp * APW + grp) * 9 * kWPad;
-  int* rl = rowl + (warp * APW + grp) * W * W;
+  float* tb = tabs + warp * 9 * kWPad;
+  int* rl = rowl + warp * W * W;
   int gjy[NG], gjz[NG];
 #pragma unroll
   for (int g = 0; g < NG; g++) {
-    const int r = g * GL + gl;
+    const int r = g * 32 + lane;
     gjz[g] = r < W * W ? r / W : 0;
     gjy[g] = r < W * W ? r - (r / W) * W : 0;
   }
-  const unsigned gmask = GL == 32 ? 0xffffffffu : ((1u << GL) - 1u);
   const double pref_sp = (double)sp.pref, inv_s2 = 2.0 * (double)sp.inv_2s2;
   const double cA = c * (double)sg.pref;
   for (int c0 = 0; c0 < natoms; c0 += kGatherList) {
@@ -573,7 +570,7 @@ __device__ __forceinline__ void adj_gather_brick(
       for (int d = 0; d < 3; d++) {
         const int cc = centre_cell(pos3[d], sp.inv_h[d]);
         loc[d] = wrap1(cc, sp.M[d]) - org[d];
-        for (int j = gl; j < W; j += GL) {
+        for (int j = lane; j < W; j += 32) {
           const float u = sub_rn(pos3[d], mul_rn((float)(cc - n + j), sp.h[d]));
           const float u2 = mul_rn(u, u);
           tb[(d * 3 + 0) * kWPad + j] = u;
@@ -600,7 +597,7 @@ __device__ __forceinline__ void adj_gather_brick(
       float P = 0.f, Vx = 0.f, Vy = 0.f, Vz = 0.f;
 #pragma unroll
       for (int g = 0; g < NG; g++) {
-        if (g * GL + gl < W * W) {
+        if (g * 32 + lane < W * W) {
           const int jy = gjy[g], jz = gjz[g];
           const float* row = tpsi + (loc[2] + jz) * ZP + (loc[1] + jy) * TP + loc[0];
           unsigned long long s0 = 0ull, s1 = 0ull;
@@ -628,13 +625,13 @@ __device__ __forceinline__ void adj_gather_brick(
       int nrow = 0;
 #pragma unroll
       for (int g = 0; g < NG; g++) {
-        const int r = g * GL + gl;
+        const int r = g * 32 + lane;
         bool ne = false;
         if (r < W * W)
           ne = add_rn(tb[(1 * 3 + 1) * kWPad + gjy[g]], tb[(2 * 3 + 1) * kWPad + gjz[g]]) <
                sg.rcut2;
-        const unsigned m = (__ballot_sync(0xffffffffu, ne) >> (GL * grp)) & gmask;
-        if (ne) rl[nrow + __popc(m & ((1u << gl) - 1u))] = (gjz[g] << 8) | gjy[g];
+        const unsigned m = __ballot_sync(0xffffffffu, ne);
+        if (ne) rl[nrow + __popc(m & ((1u << lane) - 1u))] = (gjz[g] << 8) | gjy[g];
         nrow += __popc(m);
       }
       __syncwarp();
@@ -650,7 +647,7 @@ __device__ __forceinline__ void adj_gather_brick(
       // there (rem <= rcut^2): the rows are then summed over the inner points
       const bool ends = dx2[0] < sg.rcut2 || dx2[W - 1] < sg.rcut2;
       const bool trim = !__any_sync(0xffffffffu, ends);
-      for (int i = gl; i < nrow; i += GL) {
+      for (int i = lane; i < nrow; i += 32) {
         const int r = rl[i];
         const int jz = r >> 8, jy = r & 255;
         const float uy2 = tb[(1 * 3 + 1) * kWPad + jy], uz2 = tb[(2 * 3 + 1) * kWPad + jz];

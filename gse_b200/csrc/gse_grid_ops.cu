@@ -511,16 +511,21 @@ cudaError_t launch_conv_pass(const CT* in, CT* out, const int M[3], int axis,
     const long long groups = (rows + 7) / 8;
     if (groups > 0x7fffffffLL || nruns > 65535) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)groups, nruns);
-    switch (W) {
+    // widths 5 to 15 in FP32 are conv_pass2's
+    bool done = false;
+    if constexpr (sizeof(CT) == 8) {
+      done = true;
+      switch (W) {
 #define CONV_X(WW) \
   case WW:         \
     k_conv_x_w<CT, WW><<<grid, blk, 0, st>>>(in, out, M[0], rows, run, taps); \
     break;
-      CONV_X(5) CONV_X(7) CONV_X(9) CONV_X(11) CONV_X(13) CONV_X(15)
+        CONV_X(5) CONV_X(7) CONV_X(9) CONV_X(11) CONV_X(13) CONV_X(15)
 #undef CONV_X
-      default:
-        k_conv_x<CT><<<grid, blk, 0, st>>>(in, out, M[0], rows, run, taps);
+        default: done = false;
+      }
     }
+    if (!done) k_conv_x<CT><<<grid, blk, 0, st>>>(in, out, M[0], rows, run, taps);
   } else {
     const int ma = axis == 1 ? M[1] : M[2], other = axis == 1 ? M[2] : M[1];
     const int nruns = (ma + kConvRun - 1) / kConvRun;

@@ -11,8 +11,8 @@
 //  gather    CpuGaussCharge::interpolateLoop (CpuGaussCharge.cpp:105-172): a
 //            CTA owns the atoms of a kGX x kGY x kGZ-cell brick and stages the
 //            potential of the brick plus its n-cell halo in shared memory;
-//            kGatherLanes lanes per atom, over the non-empty (y, z) rows of
-//            its sphere.
+//            kGatherLanes lanes per atom, over one list per block of the
+//            (y, z) rows that an atom's sphere can reach.
 #include <atomic>
 #include <type_traits>
 

@@ -25,9 +25,6 @@ constexpr int kScatterList = 1024;  // atoms per scatter round (per brick)
 constexpr int kGatherList = 512;    // atoms per gather round (per brick)
 constexpr int kAX = 16, kAY = 8, kAZ = 8;  // reverse-pass gather brick (two staged grids)
 constexpr int kAdjThreads = 256;           // >= kAY * kAZ
-// lanes per atom in the reverse-pass gather: a whole warp (two atoms per warp
-// would need more shared memory than two blocks per SM leave for its tables)
-constexpr int kAdjLanes = 32;
 
 // Atoms sorted by key (z cell, y cell, x bin); start[k] .. start[k+1] is bin k.
 struct BinLayout {
@@ -76,10 +73,11 @@ inline int* bin_rank(const BinScratch& w, int* perm) {
 // Few atoms in few bins are binned by one block in one launch: an atom per thread, the
 // bins in shared memory within the 48 KB that need no opt-in.  Launches bound these
 // calls; against the three or four launches of the general path an energy-force call
-// takes (FP64) 37.0 instead of 41.1 us for 2 atoms on 20^3, 49.3 / 53.4 for 300 on 20^3,
-// 65.7 / 66.7 for 1000 on 24^3, 58.8 / 57.6 on 32^3 (the nine exponentials per atom then
-// keep the one SM busy for longer than the launches saved), mixed 41.2 / 43.2 for 100 on
-// 16^3, 55.4 / 57.5 for 1000 on 24^3, 53.6 / 57.5 on 32^3.
+// takes (FP64) 37.0 instead of 41.1 us for 2 atoms on 20^3, 49.3 / 53.4 for 300 on 20^3;
+// with 1000 atoms, past the FP64 limit, it took 65.7 / 66.7 on 24^3 and 58.8 / 57.6 on 32^3
+// (the nine exponentials per atom then keep the one SM busy for longer than the launches
+// saved), which set that limit; mixed 41.2 / 43.2 for 100 on 16^3, 55.4 / 57.5 for 1000
+// on 24^3, 53.6 / 57.5 on 32^3.
 constexpr int kBinSmall = 1024;
 inline bool bin_small(bool fp64, int n, int nb) {
   return n <= (fp64 ? kBinSmall / 2 : kBinSmall) && nb <= 10240;
