@@ -789,7 +789,7 @@ cudaError_t adj_scatter_w(const float4* sorted, const float4* gs, const int* sta
   e = cudaMemsetAsync(grid64, 0, sizeof(long long) * size, st);
   if (e != cudaSuccess) return e;
   dim3 grd((b.M[0] + kSB - 1) / kSB, (b.M[1] + kSB - 1) / kSB, (b.M[2] + kSB - 1) / kSB);
-  const int nparts = scatter_parts((long long)grd.x * grd.y * grd.z);
+  const int nparts = scatter_parts((long long)grd.x * grd.y * grd.z, W);
   grd.x *= nparts;
   k_adj_scatter<W><<<grd, kAdjScatterThreads, smem, st>>>(
       sorted, gs, start, b, s, (float)(c * (double)s.pref), nparts, grid64);

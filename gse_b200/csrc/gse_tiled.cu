@@ -882,7 +882,7 @@ static cudaError_t scatter_w(const float4* sorted, const int* start, const BinLa
                              const Stencil<float>& s, long long* grid64, float* rho, bool zeroed,
                              cudaStream_t st) {
   dim3 grid((b.M[0] + kSB - 1) / kSB, (b.M[1] + kSB - 1) / kSB, (b.M[2] + kSB - 1) / kSB);
-  const int nparts = scatter_parts((long long)grid.x * grid.y * grid.z);
+  const int nparts = scatter_parts((long long)grid.x * grid.y * grid.z, W);
   grid.x *= nparts;
   if (nparts > 1)
     return scatter_shape<W, true>(sorted, start, b, s, grid, nparts, grid64, rho, zeroed, st);
