@@ -348,6 +348,7 @@ __device__ __forceinline__ void adj_scatter_brick(
   const int shift = brick_prologue<W, NT>(
       start, b, x0, y0, z0, tile, rng_a, rng_p,
       [&](int i) { return fabsf(sorted[i].w) * acA * gs[i].w; }, &total);
+  if (part * NW >= total) return;  // (uniform) as in scatter_brick
   const float tscale = exp2f((float)shift);
   // (x, z) pairs of the stencil plane each lane tests, the same for every atom
   int psxz[NPASS];  // x | z << 8

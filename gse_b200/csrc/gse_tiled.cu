@@ -286,6 +286,7 @@ __device__ __forceinline__ void scatter_brick(const float4* __restrict__ sorted,
   const int shift = brick_prologue<W, NT>(
       start, b, x0, y0, z0, tile, rng_a, rng_p,
       [&](int i) { return fabsf(sorted[i].w) * apref; }, &total);
+  if (part * NW >= total) return;  // (uniform) no atom is this block's: nothing to add
   const float tscale = exp2f((float)shift);
 
   // per-lane (x, z) pair of each pass and its tile offset: the same for all atoms
